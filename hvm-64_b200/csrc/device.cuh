@@ -48,7 +48,9 @@ constexpr int HEADROOM = HVM_HEADROOM;  // stack slots kept free for the redexes
 static_assert((SCAP & (SCAP - 1)) == 0 && SCAP >= 64, "SCAP is a power of two, at least 64");
 static_assert(HEADROOM >= 0 && SCAP - HEADROOM >= 32, "a step's window needs SCAP - HEADROOM >= 32");
 constexpr int CHUNK = 32;           // redexes per global-queue slot
-constexpr int POOL = 64;            // per-warp pool of free nodes ready for reuse
+constexpr int POOL = 96;            // per-warp pool of free nodes ready for reuse
+constexpr int FREED_ALONE = 2;      // words an interaction may have freed alone before it looks at their siblings
+constexpr int FAILS = 2;            // wires of an interaction, left as redirects, that it remembers
 constexpr unsigned ICACHE = 32;     // instructions of the step's Def staged in shared memory
 constexpr unsigned SMALL_REGS = 10; // Defs with at most this many registers use shared memory
 
@@ -87,9 +89,7 @@ struct Ctrl {
   ull stat_donated, stat_spilled, stat_overflow, stat_taken;
   ull stat_steps, stat_lanes, stat_busy_cycles, stat_idle_cycles;
   ull timeout_ns;  // per launch: each warp's deadline is its start + timeout_ns
-  ull stat_lane_sum, stat_lane_max, stat_total;  // per-lane interaction cycles (sum, per-step max), warp lifetime
-  ull stat_prof[32];  // profiling build: loads, exchanges, CAS (count, cycles), stores, per-rule cycles
-  ull pad5[16];
+  ull pad5[7];
   ull req_head;       // serving: requests admitted so far
   ull pad6[15];
   ull req_tail;       // serving: requests the host has written (host copies, device reads)
@@ -239,6 +239,7 @@ __device__ __forceinline__ unsigned smem_add_u32(unsigned* p, unsigned v) {
 // A release fence: the node fills and links before it are visible to any
 // lane that later reaches the node through a port published after it.
 __device__ __forceinline__ void mem_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void mem_fence_sc() { asm volatile("fence.sc.gpu;" ::: "memory"); }
 __device__ __forceinline__ void pause_brief() { __nanosleep(64); }
 // LOCK-fill nodes [s, s+n) with 16-byte stores.
 __device__ __forceinline__ void lock_fill(ull* H, ull s, ull n) {
@@ -294,6 +295,7 @@ inline int atom_add_i32(int* p, int v) { return std::atomic_ref<int>(*p).fetch_a
 inline int smem_add_i32(int* p, int v) { return atom_add_i32(p, v); }
 inline unsigned smem_add_u32(unsigned* p, unsigned v) { return atom_add_u32(p, v); }
 inline void mem_fence() { std::atomic_thread_fence(std::memory_order_seq_cst); }
+inline void mem_fence_sc() { std::atomic_thread_fence(std::memory_order_seq_cst); }
 inline void pause_brief() { std::this_thread::yield(); }
 inline void lock_fill(ull* H, ull s, ull n) {
   for (ull k = 0; k < 2 * n; k++) st_gpu(H + 2 * s + k, P_LOCK);
@@ -330,13 +332,35 @@ HVM_INL bool is_expand(ull p) { return ptag(p) == T_REF && (p & X_BIT) != 0; }
 // Trg (runtime/src/linker.rs:228-281): a wire is its address with the Red tag.
 HVM_INL bool trg_is_wire(ull t) { return ptag(t) == T_RED; }
 
+// The rules other than Def calls run as short instruction lists of the same
+// VM (see exec_ins), on registers their set-up fills (see classify):
+//   two links of consumed wires   registers 0, 1 (one node's words) with 2, 3
+//   four links                    registers 0 - 3 (two nodes' words) with 4 - 7
+//   a binary operator and a number: register 0 (rhs wire), 1 (result wire), 2 (number and operator)
+constexpr unsigned RULE_LINK2 = 0, RULE_LINK2_LEN = 2;
+constexpr unsigned RULE_LINK4 = 2, RULE_LINK4_LEN = 4;
+constexpr unsigned RULE_OP = 6, RULE_OP_LEN = 2;
+constexpr unsigned RULE_INS = 8;
+constexpr uint8_t I_OPRED = 9;  // do_op_num on a T_OP node's two wires (device-only instruction)
+#ifdef __CUDACC__
+__constant__
+#else
+inline
+#endif
+const DevInstr RULES[RULE_INS] = {
+    {I_LINK, 0, 0, 0, 2, 0, 0, 0}, {I_LINK, 0, 0, 1, 3, 0, INS_A_LAST | INS_B_LAST, 0},
+    {I_LINK, 0, 0, 0, 4, 0, 0, 0}, {I_LINK, 0, 0, 1, 5, 0, INS_A_LAST, 0},
+    {I_LINK, 0, 0, 2, 6, 0, 0, 0}, {I_LINK, 0, 0, 3, 7, 0, INS_A_LAST, 0},
+    {I_OPRED, 0, 0, 0, 2, 2, 0, 0}, {I_LINK, 0, 0, 1, 2, 0, INS_A_LAST, 0},
+};
+
 // Rule class of a redex, following interact()'s dispatch: the Def index for
 // a Def call (calls of one Def run the same instruction stream), else a small
 // code per rule.  Warps pick redexes of one class per step to stay convergent.
 HVM_INL unsigned redex_class(ull a, ull b) {
   unsigned at = unsigned(a & 7), bt = unsigned(b & 7);
-  if (at == T_REF && !(a & X_BIT) && a != P_ERA) return 64 + unsigned((a & A_MASK) >> 3);
-  if (bt == T_REF && !(b & X_BIT) && b != P_ERA) return 64 + unsigned((b & A_MASK) >> 3);
+  if (at == T_REF && !(a & X_BIT) && a != P_ERA) return 63 + unsigned((a & A_MASK) >> 3);  // 64 + Def index
+  if (bt == T_REF && !(b & X_BIT) && b != P_ERA) return 63 + unsigned((b & A_MASK) >> 3);
   if ((a & X_BIT) || (b & X_BIT)) return 1;
   if (at == bt) return 2 + at;  // annihilation (or nilary pair)
   return 16 + at * 8 + bt;      // commutation / native ops
@@ -351,41 +375,44 @@ struct alignas(16) WarpSmem {
   ull regs[SMALL_REGS * 32];  // VM registers, [register][lane]
   ull pool[POOL];             // free nodes ready for reuse
   ull freed[POOL];            // nodes reclaimed during the current step
-  ull sel[64];                // the redexes chosen for the current step
   DevInstr icache[ICACHE];    // the instructions of `icache_def`, staged for this step
+  DevInstr rules[RULE_INS];   // the rules' own instructions (RULES)
   DevDef idef;                // that Def's header
   unsigned icache_def;        // Def index staged in icache (~0u: none)
   ull rw[NCOUNT];             // counters of the warp's current net
   unsigned cnt[NCOUNT * 32];  // per lane: counts of this step, [counter][lane] (folded into rw)
   ull ovf[32];                // per lane: free list head | pushes since published << 48 (see free_list_push)
-  ull fw[4 * 32];             // per lane: words freed alone by the current interaction
+  ull fw[FREED_ALONE * 32];   // per lane: words freed alone by the current interaction
+  ull fails[FAILS * 32];      // per lane: consumed wires the current interaction left as redirects
   ull bnext[32], bend[32];    // per lane: pre-LOCKed bump chunk [bnext, bend), node indices
+#ifdef HVM_GEN_INCLUDE
   unsigned allocs[32];        // per lane: nodes allocated (for the DREF statistics)
+#endif
   unsigned ring_base;         // this step's pushes go to stack slots ring_base + k ...
   unsigned ring_cap;          // ... for k < ring_cap; push k >= ring_cap goes to the overflow stack
   ull* sp;                    // this warp's overflow stack in HBM (null: none; pushes go to the queue)
   ull* bigregs;               // this warp's register files for Defs above LOCAL_REGS (null: none)
   unsigned sp_n, sp_cap;      // redexes in it between steps, and its capacity
   int pool_cap;               // 0: no reuse pool (reclaimed nodes go to `ovf`)
-#ifdef HVM_PROFILE_OPS
-  ull prof[32];               // profiling build: op counts and wait cycles, cycles per rule
-#endif
-  ull st_steps, st_lanes, st_busy, st_idle, st_lane_sum, st_lane_max, st_total;
+  ull st_steps, st_lanes, st_busy, st_idle;
   unsigned ring_cnt;
   int pool_n;
   int freed_n;
   unsigned pad;
 };
-static_assert(sizeof(WarpSmem) % 16 == 0 && offsetof(WarpSmem, icache) % 16 == 0,
-              "icache of every warp's state must be 16-byte aligned");
+static_assert(sizeof(WarpSmem) % 16 == 0 && offsetof(WarpSmem, icache) % 16 == 0 &&
+                  offsetof(WarpSmem, rules) % 16 == 0 && offsetof(WarpSmem, stk) % 16 == 0,
+              "the 16-byte accesses to every warp's state must be aligned");
 
 // Initial per-lane / per-warp runtime state (lane `ln` of warp state `W`).
 HVM_INL void lane_init(WarpSmem* W, unsigned ln) {
   for (int k = 0; k < NCOUNT; k++) W->cnt[k * 32 + ln] = 0;
   W->ovf[ln] = 0;
-  for (int k = 0; k < 4; k++) W->fw[k * 32 + ln] = 0;
+  for (int k = 0; k < FREED_ALONE; k++) W->fw[k * 32 + ln] = 0;
   W->bnext[ln] = W->bend[ln] = 0;
+#ifdef HVM_GEN_INCLUDE
   W->allocs[ln] = 0;
+#endif
 }
 
 // ---- cold paths as free functions over scalars -------------------------------
@@ -481,9 +508,13 @@ HVM_COLD void free_publish(unsigned net, ull* ovf) {
   *ovf = 0;
 }
 // Take one batch from the shared stack as the lane's list; false when empty.
+// (The lanes of a step run out together and contend for the top: each lost
+// CAS is another lane's success, so a lane tries long enough for many of
+// them before it falls back to fresh nodes.)
 HVM_COLD bool free_take(unsigned net, ull* ovf) {
   ull* top = &g_P.ctrl->free_top;
-  for (int tries = 0; tries < 64; tries++) {
+  for (int tries = 0; tries < 2048; tries++) {
+    if ((tries & 7) == 7) pause_brief();
     ull t = ld_gpu(top);
     ull a = t & FT_ADDR;
     if (a == 0) return false;
@@ -506,6 +537,11 @@ struct Refill {
 HVM_COLD Refill alloc_refill(unsigned net, ull* ovf) {
   if ((*ovf & OVF_ADDR) != 0 || (past_reuse_mark() && free_take(net, ovf))) {
     ull a = *ovf & OVF_ADDR, n = *ovf >> 48;
+    if (a >= g_P.heap_bytes) {  // links are heap words: checked before the node is handed out
+      run_fail(net, HVM64_ERR_BAD_ADDR, a);
+      *ovf = 0;
+      return {0, 0, 0};
+    }
     *ovf = (ld_gpu(heap_at(net, a)) & OVF_ADDR) | ((n ? n - 1 : 0) << 48);
     st_gpu(heap_at(net, a), P_LOCK);
     mem_fence();
@@ -544,49 +580,14 @@ struct Ctx {
 #define LS(field) (c.W->field[c.lane])             // a lane's slot
 #define FW(k) (c.W->fw[(k) * 32 + c.lane])          // freed-word slot k
 
-HVM_INL ull hload(const Ctx& c, ull a) {
-#if defined(HVM_PROFILE_OPS) && defined(__CUDACC__)
-  long long t = clock64();
-  ull v = ld_gpu(heap_at(c.net, a));
-  asm volatile("" : "+l"(v));
-  atomicAdd(&c.W->prof[0], 1ull);
-  atomicAdd(&c.W->prof[1], ull(clock64() - t));
-  return v;
-#else
-  return ld_gpu(heap_at(c.net, a));
-#endif
-}
-#if defined(HVM_PROFILE_OPS) && defined(__CUDACC__)
-HVM_INL ull prof_done(const Ctx& c, int k, long long t, ull v) {
-  asm volatile("" : "+l"(v));
-  atomicAdd(&c.W->prof[k], 1ull);
-  atomicAdd(&c.W->prof[k + 1], ull(clock64() - t));
-  return v;
-}
-HVM_INL void hstore(const Ctx& c, ull a, ull v) {
-  atomicAdd(&c.W->prof[6], 1ull);
-  st_gpu(heap_at(c.net, a), v);
-}
-HVM_INL ull hswap(const Ctx& c, ull a, ull v) {
-  long long t = clock64();
-  return prof_done(c, 2, t, atom_exch(heap_at(c.net, a), v));
-}
-HVM_INL ull hcas(const Ctx& c, ull a, ull e, ull v) {
-  long long t = clock64();
-  return prof_done(c, 4, t, atom_cas(heap_at(c.net, a), e, v));
-}
-#define PROF_RULE(idx) long long prof_t0 = clock64(); struct ProfEnd { const Ctx& c; long long t; int k; \
-  __device__ ~ProfEnd() { atomicAdd(&c.W->prof[8 + 2 * k], 1ull); atomicAdd(&c.W->prof[9 + 2 * k], ull(clock64() - t)); } } prof_end{c, prof_t0, idx};
-#else
-HVM_INL void hstore(const Ctx& c, ull a, ull v) { st_gpu(heap_at(c.net, a), v); }
-HVM_INL ull hswap(const Ctx& c, ull a, ull v) { return atom_exch(heap_at(c.net, a), v); }
-HVM_INL ull hcas(const Ctx& c, ull a, ull e, ull v) { return atom_cas(heap_at(c.net, a), e, v); }
-#define PROF_RULE(k)
-#endif
-HVM_INL void count(const Ctx& c, int k, ull v = 1) { c.W->cnt[k * 32 + c.lane] += unsigned(v); }
+HVM_INL ull hload(const Ctx c, ull a) { return ld_gpu(heap_at(c.net, a)); }
+HVM_INL void hstore(const Ctx c, ull a, ull v) { st_gpu(heap_at(c.net, a), v); }
+HVM_INL ull hswap(const Ctx c, ull a, ull v) { return atom_exch(heap_at(c.net, a), v); }
+HVM_INL ull hcas(const Ctx c, ull a, ull e, ull v) { return atom_cas(heap_at(c.net, a), e, v); }
+HVM_INL void count(const Ctx c, int k, ull v = 1) { c.W->cnt[k * 32 + c.lane] += unsigned(v); }
 
 // wire.rs:342-350
-HVM_INL ull lock_target(const Ctx& c, ull w) {
+HVM_INL ull lock_target(const Ctx c, ull w) {
   ull got = hswap(c, w, P_LOCK);
   return got != P_LOCK ? got : relock(c.net, w);
 }
@@ -594,24 +595,38 @@ HVM_INL ull lock_target(const Ctx& c, ull w) {
 // ---- allocator -------------------------------------------------------------
 // The reference's allocator (runtime/src/allocator.rs:73-110) writes LOCK
 // into both words of every node it hands out and links a node into a free
-// list once both halves are FREE.  Here a node is LOCK-filled when it becomes
-// free (or when its bump chunk is taken) and that fill is fenced before the
-// node is handed out again, so alloc() itself touches no heap memory.  A node
-// whose two halves are both freed by the same interaction is reclaimed
-// without reading the other half; otherwise the reference's store-FREE /
-// read-other-half / CAS sequence decides which lane reclaims.
-HVM_COLD void recycle(const Ctx& c, ull node) {
+// list once both halves are FREE.  Here a free node always holds LOCK in both
+// words, so alloc() itself touches no heap memory:
+//  - a bump chunk is LOCK-filled and fenced when it is taken;
+//  - a node an interaction consumes has both its words taken by exchanges
+//    with LOCK.  Once both wires are linked nothing refers to the node, it
+//    already holds what a free node must hold, and it is reclaimed without
+//    touching memory (recycle; see wire_done);
+//  - a word freed alone follows the reference's store-FREE / read-other-half /
+//    CAS sequence, which decides which lane reclaims the node (half_free,
+//    settle, claim); the lane that does writes LOCK and fences.
+// Every address alloc() returns lies in the heap: it comes from the bump
+// pointer, from recycle() (called with checked addresses), or from a list
+// whose links are checked as they are followed (alloc_refill).  Stores to a
+// new node's words therefore need no check of their own, even in the steps
+// that still run after an allocation failed (alloc() then returns node 0, a
+// scratch node).
+HVM_COLD void recycle_spill(const Ctx c, ull node) { free_list_push(c.net, &LS(ovf), node); }
+HVM_INL void recycle(const Ctx c, ull node) {
 #ifdef HVM_EMU_CHECK_ALLOC
   check_reclaimed(node);
 #endif
   int k = c.W->pool_cap ? smem_add_i32(&c.W->freed_n, 1) : POOL;
-  if (k < c.W->pool_cap) {
-    c.W->freed[k] = node;
-  } else {
-    free_list_push(c.net, &LS(ovf), node);  // right word already LOCK
-  }
+  if (k < c.W->pool_cap) c.W->freed[k] = node;
+  else recycle_spill(c, node);
 }
-HVM_COLD ull alloc_slow(const Ctx& c) {
+// A node whose words this lane has just LOCKed with stores.
+HVM_COLD void recycle_stored(const Ctx c, ull node) {
+  if (node >= g_P.heap_bytes) return run_fail(c.net, HVM64_ERR_BAD_ADDR, node);
+  mem_fence();  // the LOCKs are visible before the node is handed out again
+  recycle(c, node);
+}
+HVM_COLD ull alloc_slow(const Ctx c) {
   Refill r = alloc_refill(c.net, &LS(ovf));
   if (r.bend) {
     LS(bnext) = r.bnext;
@@ -620,17 +635,19 @@ HVM_COLD ull alloc_slow(const Ctx& c) {
   return r.node;
 }
 #ifdef HVM_EMU_CHECK_ALLOC
-HVM_INL ull alloc_unchecked(const Ctx& c);
-HVM_INL ull alloc(const Ctx& c) {
+HVM_INL ull alloc_unchecked(const Ctx c);
+HVM_INL ull alloc(const Ctx c) {
   ull n = alloc_unchecked(c);
   check_handed_out(n);
   return n;
 }
-HVM_INL ull alloc_unchecked(const Ctx& c) {
+HVM_INL ull alloc_unchecked(const Ctx c) {
 #else
-HVM_INL ull alloc(const Ctx& c) {
+HVM_INL ull alloc(const Ctx c) {
 #endif
+#ifdef HVM_GEN_INCLUDE
   LS(allocs)++;
+#endif
   if (c.W->pool_cap) {
     int k = smem_add_i32(&c.W->pool_n, -1) - 1;
     if (k >= 0) return c.W->pool[k];
@@ -642,70 +659,64 @@ HVM_INL ull alloc(const Ctx& c) {
   }
   return alloc_slow(c);
 }
+HVM_COLD ull alloc_cold(const Ctx c) { return alloc(c); }
 // A word freed alone: a node found fully free is claimed by CAS on its left
 // word, then kept only if its right word is still free -- between the load
 // and the CAS the node may have been reclaimed by the other half's owner,
 // reused, and half-freed again (ABA); then the left word is handed back.
-HVM_COLD void claim(const Ctx& c, ull w, ull other) {
+HVM_COLD void claim(const Ctx c, ull w, ull other) {
   if (!w || other != P_FREE) return;
   ull l = w & ~8ull;
   if (hcas(c, l, P_FREE, P_LOCK) != P_FREE) return;
   if (hload(c, l | 8) == P_FREE) {
     hstore(c, l | 8, P_LOCK);
-    recycle(c, l);
+    recycle_stored(c, l);
   } else {
     hstore(c, l, P_FREE);
   }
 }
 // End of an interaction: look at the other half of every word freed alone
 // (the loads are in flight together).
-HVM_COLD void settle(const Ctx& c) {
-  PROF_RULE(6)
-  ull w0 = FW(0), w1 = FW(1), w2 = FW(2), w3 = FW(3);
-  if (!(w0 | w1 | w2 | w3)) return;
+HVM_COLD void settle(const Ctx c) {
+  ull w0 = FW(0), w1 = FW(1);
+  if (!(w0 | w1)) return;
+  mem_fence_sc();  // the FREEs are visible before the loads: of two lanes freeing one node's halves, one sees both
   ull o0 = w0 ? hload(c, w0 ^ 8) : 0, o1 = w1 ? hload(c, w1 ^ 8) : 0;
-  ull o2 = w2 ? hload(c, w2 ^ 8) : 0, o3 = w3 ? hload(c, w3 ^ 8) : 0;
-  FW(0) = FW(1) = FW(2) = FW(3) = 0;
+  FW(0) = FW(1) = 0;
   claim(c, w0, o0);
   claim(c, w1, o1);
-  claim(c, w2, o2);
-  claim(c, w3, o3);
 }
-HVM_COLD void half_free(const Ctx& c, ull a) {
-  PROF_RULE(8)
+HVM_COLD void half_free(const Ctx c, ull a) {
   ull x = a ^ 8;
   int k = -1;
   if (a != 0) {
     if (FW(0) == x) k = 0;
     else if (FW(1) == x) k = 1;
-    else if (FW(2) == x) k = 2;
-    else if (FW(3) == x) k = 3;
   }
   if (k >= 0) {  // both halves freed by this interaction: no one else can claim the node
     FW(k) = 0;
     ull l = a & ~8ull;
     hstore(c, l, P_LOCK);
     hstore(c, l | 8, P_LOCK);
-    recycle(c, l);
+    recycle_stored(c, l);
     return;
   }
   hstore(c, a, P_FREE);
   if (FW(0) == 0) FW(0) = a;
   else if (FW(1) == 0) FW(1) = a;
-  else if (FW(2) == 0) FW(2) = a;
-  else if (FW(3) == 0) FW(3) = a;
   else {
     settle(c);
     FW(0) = a;
   }
 }
+static_assert(FREED_ALONE == 2, "settle and half_free name their slots");
 
 // ---- redex pushes (linker.rs:70-85) -----------------------------------------
 // The reference's queue is an unbounded vector (linker.rs:308-344); here a
 // step's k-th push goes to the warp's shared-memory stack while it has room,
 // then to the warp's private overflow stack in HBM (slot sp_n + k - ring_cap),
 // then to the global queue.  None of these waits for anyone.
-HVM_COLD void push_spill(const Ctx& c, ull a, ull b, unsigned j) {
+HVM_COLD void push_spill(const Ctx c, ull a, ull b, unsigned j) {
   unsigned i = c.W->sp_n + j;
   if (c.W->sp && i < c.W->sp_cap) {
     c.W->sp[2 * ull(i)] = a;
@@ -714,7 +725,7 @@ HVM_COLD void push_spill(const Ctx& c, ull a, ull b, unsigned j) {
   }
   push_overflow(c.net, a, b);
 }
-HVM_INL void push(const Ctx& c, ull a, ull b) {
+HVM_INL void push(const Ctx c, ull a, ull b) {
   unsigned cap = c.W->ring_cap;
   unsigned k = smem_add_u32(&c.W->ring_cnt, 1u);
   if (k < cap) {
@@ -744,16 +755,16 @@ HVM_INL unsigned pushes_bound(unsigned cls) {
   }
   return 4;
 }
-HVM_INL void redux(const Ctx& c, ull a, ull b) {
+HVM_INL void redux(const Ctx c, ull a, ull b) {
   if (skippable(a) && skippable(b)) count(c, RW_ERAS);
   else push(c, a, b);
 }
 
 // ---- linker (runtime/src/linker.rs:25-203) ----------------------------------
-HVM_INL void half_link_port_port(const Ctx& c, ull a, ull b) {
+HVM_INL void half_link_port_port(const Ctx c, ull a, ull b) {
   if (ptag(a) == T_VAR) hstore(c, paddr(a), b);
 }
-HVM_INL void link_port_port(const Ctx& c, ull a, ull b) {
+HVM_INL void link_port_port(const Ctx c, ull a, ull b) {
   if (principal(a) && principal(b)) {
     redux(c, a, b);
   } else {
@@ -761,10 +772,10 @@ HVM_INL void link_port_port(const Ctx& c, ull a, ull b) {
     half_link_port_port(c, b, a);
   }
 }
-HVM_COLD void resolve_redirect_pri(const Ctx& c, ull ap, ull aw, ull bp);
+HVM_COLD void resolve_redirect_pri(const Ctx c, ull ap, ull aw, ull bp);
 // The CAS lost against another lane linking the same wire: leave a redirect
 // (linker.rs:109-123).
-HVM_COLD void half_link_failed(const Ctx& c, ull ap, ull aw, ull bp) {
+HVM_COLD void half_link_failed(const Ctx c, ull ap, ull aw, ull bp) {
   if (ptag(bp) == T_VAR) {
     hstore(c, aw, pred(paddr(bp)));
   } else if (principal(bp)) {
@@ -774,7 +785,7 @@ HVM_COLD void half_link_failed(const Ctx& c, ull ap, ull aw, ull bp) {
     run_fail(c.net, HVM64_ERR_BAD_PAIR, bp);
   }
 }
-HVM_COLD void half_link_wire_port(const Ctx& c, ull ap, ull aw, ull bp) {
+HVM_COLD void half_link_wire_port(const Ctx c, ull ap, ull aw, ull bp) {
   if (ptag(ap) == T_VAR) {
     if (hcas(c, paddr(ap), pvar(aw), bp) == pvar(aw)) half_free(c, aw);
     else half_link_failed(c, ap, aw, bp);
@@ -782,8 +793,7 @@ HVM_COLD void half_link_wire_port(const Ctx& c, ull ap, ull aw, ull bp) {
     half_free(c, aw);
   }
 }
-HVM_COLD void link_wire_wire(const Ctx& c, ull aw, ull bw) {
-  PROF_RULE(9)
+HVM_COLD void link_wire_wire(const Ctx c, ull aw, ull bw) {
   // Both words belong to nodes this interaction consumes, so no other lane
   // takes them: the two exchanges go out together (one round trip instead of
   // two) and give the values the reference's take-one-then-the-other does; a
@@ -802,8 +812,7 @@ HVM_COLD void link_wire_wire(const Ctx& c, ull aw, ull bw) {
   }
 }
 // link_wire_port for a wire whose target `ap` was already taken (locked).
-HVM_COLD void link_locked_wire_port(const Ctx& c, ull aw, ull ap, ull bp) {
-  PROF_RULE(10)
+HVM_COLD void link_locked_wire_port(const Ctx c, ull aw, ull ap, ull bp) {
   if (principal(ap) && principal(bp)) {
     half_free(c, aw);
     redux(c, ap, bp);
@@ -812,8 +821,8 @@ HVM_COLD void link_locked_wire_port(const Ctx& c, ull aw, ull ap, ull bp) {
     half_link_port_port(c, bp, ap);
   }
 }
-HVM_INL void link_wire_port(const Ctx& c, ull aw, ull bp) { link_locked_wire_port(c, aw, lock_target(c, aw), bp); }
-HVM_COLD void resolve_redirect_pri(const Ctx& c, ull ap, ull aw, ull bp) {
+HVM_INL void link_wire_port(const Ctx c, ull aw, ull bp) { link_locked_wire_port(c, aw, lock_target(c, aw), bp); }
+HVM_COLD void resolve_redirect_pri(const Ctx c, ull ap, ull aw, ull bp) {
   unsigned it = 0;
   for (;;) {
     ull tw = paddr(ap);
@@ -823,6 +832,7 @@ HVM_COLD void resolve_redirect_pri(const Ctx& c, ull ap, ull aw, ull bp) {
       continue;
     }
     if (ptag(tp) == T_RED) {
+      if (!run_spin(c.net, it)) return;  // (a chain of redirects is finite, but after a failure it may be a cycle)
       half_free(c, tw);
       ap = tp;
       continue;
@@ -838,6 +848,11 @@ HVM_COLD void resolve_redirect_pri(const Ctx& c, ull ap, ull aw, ull bp) {
           tp = hload(c, tw);
           if (!run_spin(c.net, it2)) return;
         }
+        // The other end's way here is cut (its word holds bp now) and every
+        // redirect on it is freed: when it led back to aw, nothing names aw
+        // any more.  (Lanes of one step often take both ends of a wire at
+        // the same time; without this each such meeting lost a node.)
+        if (tw == aw) half_free(c, aw);
         return;
       }
       if (!run_spin(c.net, it)) return;
@@ -863,104 +878,36 @@ HVM_COLD void resolve_redirect_pri(const Ctx& c, ull ap, ull aw, ull bp) {
     return;
   }
 }
-// Trg (linker.rs:228-304): a wire is its address with the Red tag.
-HVM_INL void link_trg_port(const Ctx& c, ull a, ull b) {
+// ---- compiled Defs (HVM_GEN_INCLUDE) -----------------------------------------
+// The primitives generated Def functions call: each instruction as one
+// function, freeing consumed wires word by word (half_free).
+#ifdef HVM_GEN_INCLUDE
+HVM_INL void link_trg_port(const Ctx c, ull a, ull b) {
   if (trg_is_wire(a)) link_wire_port(c, a, b);
   else link_port_port(c, a, b);
 }
-HVM_COLD void link_trg(const Ctx& c, ull a, ull b) {
+HVM_COLD void link_trg(const Ctx c, ull a, ull b) {
   bool aw = trg_is_wire(a), bw = trg_is_wire(b);
   if (aw && bw) link_wire_wire(c, a, b);
   else if (aw) link_wire_port(c, a, b);
   else if (bw) link_wire_port(c, b, a);
   else link_port_port(c, a, b);
 }
-HVM_INL void free_trg(const Ctx& c, ull t) {
+HVM_INL void free_trg(const Ctx c, ull t) {
   if (trg_is_wire(t)) half_free(c, t);
 }
 // The target of a Trg about to be consumed by a VM instruction.  A wire is
 // locked rather than read: every path of the instruction then either frees
 // that wire or links it at once (which would lock it first), so taking the
 // lock up front saves a round trip and changes nothing observable.
-HVM_INL ull trg_take(const Ctx& c, ull t) { return trg_is_wire(t) ? lock_target(c, t) : t; }
+HVM_INL ull trg_take(const Ctx c, ull t) { return trg_is_wire(t) ? lock_target(c, t) : t; }
 // link_trg_port for a Trg taken with trg_take.
-HVM_INL void link_taken(const Ctx& c, ull t, ull target, ull b) {
+HVM_INL void link_taken(const Ctx c, ull t, ull target, ull b) {
   if (trg_is_wire(t)) link_locked_wire_port(c, t, target, b);
   else link_port_port(c, t, b);
 }
 
-// ---- rules (runtime/src/interact.rs) ------------------------------------------
-HVM_COLD void anni2(const Ctx& c, ull a, ull b) {  // interact.rs:72-79
-  PROF_RULE(0)
-  count(c, RW_ANNI);
-  ull a1 = paddr(a), b1 = paddr(b);
-  link_wire_wire(c, a1, b1);
-  link_wire_wire(c, a1 ^ 8, b1 ^ 8);
-}
-HVM_COLD void comm22(const Ctx& c, ull a, ull b) {  // interact.rs:118-141
-  PROF_RULE(1)
-  count(c, RW_COMM);
-  count(c, EX_COMM22);
-  ull a1 = paddr(a), b1 = paddr(b);
-  ull A1 = alloc(c), A2 = alloc(c), B1 = alloc(c), B2 = alloc(c);
-  unsigned ta = ptag(a), la = plab(a), tb = ptag(b), lb = plab(b);
-  link_port_port(c, pvar(A1), pvar(B1));
-  link_port_port(c, pvar(A1 ^ 8), pvar(B2));
-  link_port_port(c, pvar(A2), pvar(B1 ^ 8));
-  link_port_port(c, pvar(A2 ^ 8), pvar(B2 ^ 8));
-  link_wire_port(c, a1, mkport(tb, lb, B1));
-  link_wire_port(c, a1 ^ 8, mkport(tb, lb, B2));
-  link_wire_port(c, b1, mkport(ta, la, A1));
-  link_wire_port(c, b1 ^ 8, mkport(ta, la, A2));
-}
-HVM_COLD void comm02(const Ctx& c, ull a, ull b) {  // interact.rs:162-168
-  PROF_RULE(2)
-  count(c, RW_COMM);
-  ull b1 = paddr(b);
-  link_wire_port(c, b1, a);
-  link_wire_port(c, b1 ^ 8, a);
-}
-HVM_COLD void switch_num(const Ctx& c, ull a, ull b) {  // interact.rs:201-223
-  PROF_RULE(3)
-  count(c, RW_OPER);
-  ull a1 = paddr(a);
-  uint32_t num = uint32_t(b);
-  uint32_t n = num_tag(num) == NT_U24 ? num_payload(num) : 0;
-  if (n == 0) {
-    ull x = alloc(c);
-    link_port_port(c, pvar(x ^ 8), P_ERA);
-    link_wire_port(c, a1 ^ 8, pvar(x));
-    link_wire_port(c, a1, mkport(T_CTR, 0, x));
-  } else {
-    ull x = alloc(c), y = alloc(c);
-    link_port_port(c, pvar(x), P_ERA);
-    link_port_port(c, pvar(x ^ 8), mkport(T_CTR, 0, y));
-    link_port_port(c, pvar(y), ull(num_u24(n - 1)));
-    link_wire_port(c, a1 ^ 8, pvar(y ^ 8));
-    link_wire_port(c, a1, mkport(T_CTR, 0, x));
-  }
-}
-HVM_COLD void op_num(const Ctx& c, ull a, ull b) {  // interact.rs:251-270
-  PROF_RULE(4)
-  uint32_t op = plab(a);
-  ull a1 = paddr(a);
-  ull t1 = hload(c, a1);
-  if (ptag(t1) == T_NUM) {
-    count(c, RW_OPER);
-    half_free(c, a1);
-    ull out = binary_op(c.net, uint32_t(b), op, uint32_t(t1));
-    link_wire_port(c, a1 ^ 8, out);
-  } else {
-    ull x = alloc(c);
-    link_port_port(c, pvar(x), ull(num_unary(op, uint32_t(b))));
-    link_wire_port(c, a1 ^ 8, pvar(x ^ 8));
-    link_wire_port(c, a1, mkport(T_OP, NT_SYM, x));
-  }
-}
-
-// ---- instruction VM (runtime/src/instruction.rs:400-500, def.rs:217-289) -----
-HVM_COLD void do_ctr(const Ctx& c, unsigned lab, ull trg, ull& o1, ull& o2) {
-  PROF_RULE(11)
+HVM_COLD void do_ctr(const Ctx c, unsigned lab, ull trg, ull& o1, ull& o2) {
   ull port = trg_take(c, trg);
   if (ptag(port) == T_CTR && plab(port) == lab) {
     free_trg(c, trg);
@@ -974,7 +921,7 @@ HVM_COLD void do_ctr(const Ctx& c, unsigned lab, ull trg, ull& o1, ull& o2) {
   o1 = pvar(n);
   o2 = pvar(n ^ 8);
 }
-HVM_COLD void do_op(const Ctx& c, unsigned op, ull trg, ull& o1, ull& o2) {
+HVM_COLD void do_op(const Ctx c, unsigned op, ull trg, ull& o1, ull& o2) {
   ull port = trg_take(c, trg);
   if (ptag(port) == T_NUM) {
     free_trg(c, trg);
@@ -994,7 +941,7 @@ HVM_COLD void do_op(const Ctx& c, unsigned op, ull trg, ull& o1, ull& o2) {
   o1 = pvar(n);
   o2 = pvar(n ^ 8);
 }
-HVM_COLD ull do_op_num(const Ctx& c, unsigned op, ull trg, uint32_t rhs) {
+HVM_COLD ull do_op_num(const Ctx c, unsigned op, ull trg, uint32_t rhs) {
   ull port = trg_take(c, trg);
   if (ptag(port) == T_NUM) {
     count(c, RW_OPER);
@@ -1010,13 +957,13 @@ HVM_COLD ull do_op_num(const Ctx& c, unsigned op, ull trg, uint32_t rhs) {
   hstore(c, n, ull(rhs));
   return pvar(n ^ 8);
 }
-HVM_COLD ull create_wire_to(const Ctx& c, ull port) {  // node.rs:176-182
+HVM_COLD ull create_wire_to(const Ctx c, ull port) {  // node.rs:176-182
   ull a = alloc(c);
   half_free(c, a ^ 8);
   link_port_port(c, port, pvar(a));
   return a;
 }
-HVM_COLD void do_switch(const Ctx& c, ull trg, ull& o1, ull& o2) {
+HVM_COLD void do_switch(const Ctx c, ull trg, ull& o1, ull& o2) {
   ull port = trg_take(c, trg);
   if (ptag(port) == T_NUM) {
     count(c, RW_OPER);
@@ -1049,73 +996,266 @@ HVM_COLD void do_switch(const Ctx& c, ull trg, ull& o1, ull& o2) {
   o1 = pvar(m);
   o2 = pvar(m ^ 8);
 }
-// Runs a Def's instruction list over a register file (base + i * stride).
+#endif
+
+HVM_COLD void comm02(const Ctx c, ull a, ull b) {  // interact.rs:162-168
+  count(c, RW_COMM);
+  ull b1 = paddr(b);
+  link_wire_port(c, b1, a);
+  link_wire_port(c, b1 ^ 8, a);
+}
 // An inert Def's call (transform/src/pre_reduce.rs:96-101): the redex is
 // recorded for the host, which puts it back into the net's redexes.
-HVM_COLD void capture(const Ctx& c, ull port, ull trg) {
+HVM_COLD void capture(const Ctx c, ull port, ull trg) {
   ull k = atom_add(&g_P.ctrl->captured, 1ull);
   if (k >= g_P.capture_cap) return run_fail(c.net, HVM64_ERR_OUTPUT, k);
   g_P.capture[2 * k] = port;
   g_P.capture[2 * k + 1] = trg;
 }
-HVM_COLD void exec(const Ctx& c, const DevDef& d, ull t0, ull* R, unsigned stride, const DevInstr* ins) {
-  R[0] = t0;
-  for (unsigned k = 0; k < d.ins_len; k++) {
-    const DevInstr I = ins[k];
-    ull* ra = R + I.a * stride;
-    switch (I.k) {
-      case I_CONST: *ra = I.port; break;
-      case I_LINK: count(c, EX_DLINKS); link_trg(c, *ra, R[I.b * stride]); break;
-      case I_LINKCONST: count(c, EX_DLINKS); link_trg_port(c, *ra, I.port); break;
-      case I_CTR: do_ctr(c, I.lab, *ra, R[I.b * stride], R[I.c * stride]); break;
-      case I_OP: do_op(c, I.op, *ra, R[I.b * stride], R[I.c * stride]); break;
-      case I_OPNUM: R[I.c * stride] = do_op_num(c, I.op, *ra, uint32_t(I.port)); break;
-      case I_SWITCH: do_switch(c, *ra, R[I.b * stride], R[I.c * stride]); break;
-      case I_WIRES: {
-        ull a = alloc(c);
-        R[I.a * stride] = pvar(a);
-        R[I.b * stride] = a;
-        R[I.c * stride] = pvar(a ^ 8);
-        R[I.d * stride] = a ^ 8;
-        break;
-      }
-      case I_CAPTURE: capture(c, I.port, *ra); break;
-    }
+// ---- instruction VM (runtime/src/instruction.rs:400-500, def.rs:217-289) -----
+// One function runs every instruction kind and, through the RULES lists, every
+// rule that rewires two binary nodes.  What bounds it is not memory bandwidth
+// but instruction supply and the chain of dependent L2 round trips, so it is
+// written to be inlined once into the reducer's step, without calls on its
+// usual paths (an out-of-line function per primitive spent most of its
+// instructions saving and restoring registers), and all kinds share one code
+// path for taking a wire, allocating, and linking: the lanes of a step stay
+// together and their memory operations go out together.
+//
+// Every instruction has the same shape:
+//   take    its operands that are wires, with one exchange each (both in
+//           flight together).  Every path then links or frees them at once,
+//           which would lock them first, so taking them up front changes
+//           nothing observable;
+//   rule    constructor match, operator, switch: what the operand meets;
+//   link    the operand's target with the other side (linker.rs:25-203).
+//
+// Wires an interaction consumes come in pairs, the two words of one consumed
+// node.  The encoder marks the operand that consumes the later one of a pair
+// (INS_A_LAST, INS_B_LAST); the node is reclaimed there, when neither of its
+// words was left as a redirect (wire_done, wire_failed).
+struct Exec {
+  unsigned nf = 0;  // wires left as redirects so far (the first FAILS of them are in WarpSmem::fails)
+  unsigned anni = 0, oper = 0, eras = 0, nodes = 0;
+};
+#define FAIL(k) (c.W->fails[(k) * 32 + c.lane])
+// Whether this interaction left `w` as a redirect: 1 yes, 0 no, -1 not known
+// (more redirects than are remembered).
+HVM_INL int was_failed(const Ctx c, ull w, unsigned nf) {
+  for (unsigned k = 0; k < unsigned(FAILS) && k < nf; k++)
+    if (FAIL(k) == w) return 1;
+  return nf > unsigned(FAILS) ? -1 : 0;
+}
+// The later wire of a pair was linked, and some wire of this interaction was
+// left as a redirect.
+HVM_COLD void pair_done(const Ctx c, ull w, unsigned nf) {
+  int f = was_failed(c, w ^ 8, nf);
+  if (f == 0) recycle(c, w & ~8ull);
+  else if (f == 1) half_free(c, w);  // freed alone; whoever follows the redirect frees the other half
+}  // (not known: the node is given up rather than handed out twice)
+HVM_INL void wire_done(const Ctx c, Exec& x, ull w, bool last) {
+  if (last) {
+    if (x.nf == 0) recycle(c, w & ~8ull);
+    else pair_done(c, w, x.nf);
   }
 }
-HVM_COLD void exec_large(const Ctx& c, const DevDef& d, ull t0) {
+// The CAS on wire `w`'s other end lost: leave a redirect in `w`.
+HVM_COLD void wire_failed(const Ctx c, ull xp, ull w, ull yp, unsigned nf, bool last) {
+  half_link_failed(c, xp, w, yp);
+  if (!last) {
+    if (nf < unsigned(FAILS)) FAIL(nf) = w;
+  } else if (was_failed(c, w ^ 8, nf) == 0) {
+    half_free(c, w ^ 8);  // the earlier wire was linked: its word is freed alone
+  }
+}
+#undef FAIL
+
+// Instruction `I` on registers R[i * S].
+template <unsigned S> HVM_INL void exec_ins(const Ctx c, Exec& x, const DevInstr I, ull* R) {
+  const unsigned kind = I.k;
+  if (kind == I_CONST) {
+    R[I.a * S] = I.port;
+    return;
+  }
+  if (kind == I_WIRES) {
+    ull n = alloc_cold(c);
+    x.nodes++;
+    R[I.a * S] = pvar(n);
+    R[I.b * S] = n;
+    R[I.c * S] = pvar(n ^ 8);
+    R[I.d * S] = n ^ 8;
+    return;
+  }
+  if (kind == I_CAPTURE) return capture(c, I.port, R[I.a * S]);
+  // take
+  const bool isl = kind == I_LINK;
+  const ull A = R[I.a * S];
+  const ull B = isl || kind == I_OPRED ? R[I.b * S] : I.port;
+  const bool aw = ptag(A) == T_RED, bw = isl && ptag(B) == T_RED;
+  ull ap = A, bp = B;
+  // (wires hold checked addresses: a constructor match checks its node's)
+  if (aw) ap = atom_exch(g_P.heap + (A >> 3), P_LOCK);
+  if (bw) bp = atom_exch(g_P.heap + (B >> 3), P_LOCK);
+  if (aw && ap == P_LOCK) ap = relock(c.net, A);
+  if (bw && bp == P_LOCK) bp = relock(c.net, B);
+  // rule
+  bool link = true;
+  if (kind >= I_CTR) {
+    const unsigned t = ptag(ap);
+    const bool num = t == T_NUM, match = kind == I_CTR && t == T_CTR && plab(ap) == I.lab;
+    const bool era = ap == P_ERA && kind != I_CTR && kind != I_OPRED;
+    ull n = 0, o1, o2;
+    // (an operator's result on numbers needs no node, nor does an erased one)
+    const bool fast = match || era || (num && (kind == I_OPNUM || kind == I_OPRED));
+    if (!fast) {
+      n = alloc(c);
+      x.nodes++;
+    }
+    o1 = pvar(n);
+    o2 = pvar(n ^ 8);
+    link = !fast;
+    if (kind == I_CTR) {
+      if (match) {
+        x.anni++;
+        o1 = paddr(ap);  // Trg::wire
+        if (o1 >= g_P.heap_bytes) {
+          run_fail_here(HVM64_ERR_BAD_ADDR);
+          o1 = 0;
+        }
+        o2 = o1 ^ 8;
+      }
+      bp = mkport(T_CTR, I.lab, n);
+    } else if (kind == I_SWITCH) {
+      bp = mkport(T_SWITCH, 0, n);
+      if (num) {
+        x.oper++;
+        link = false;
+        const uint32_t v = uint32_t(ap);
+        const uint32_t k = num_tag(v) == NT_U24 ? num_payload(v) : 0;
+        o1 = mkport(T_CTR, 0, n);
+        // The arms' node may be matched by the next instruction, so the
+        // word behind the result is filled now: with a wire of a node of its
+        // own (node.rs:176-182), whose other word counts as consumed.
+        ull tgt = n, w = alloc_cold(c);
+        x.nodes++;
+        if (k == 0) {
+          st_gpu(g_P.heap + ((n ^ 8) >> 3), P_ERA);
+        } else {
+          ull n2 = alloc_cold(c);
+          x.nodes++;
+          st_gpu(g_P.heap + (n >> 3), P_ERA);
+          st_gpu(g_P.heap + ((n ^ 8) >> 3), mkport(T_CTR, 0, n2));
+          st_gpu(g_P.heap + (n2 >> 3), ull(num_u24(k - 1)));
+          tgt = n2 ^ 8;
+        }
+        st_gpu(g_P.heap + (tgt >> 3), pvar(w));
+        st_gpu(g_P.heap + (w >> 3), pvar(tgt));
+        o2 = w;
+      } else if (era) {
+        x.eras++;
+        o1 = o2 = P_ERA;
+      }
+    } else if (kind == I_OP) {
+      bp = mkport(T_OP, I.op, n);
+      if (num) {
+        link = false;
+        st_gpu(g_P.heap + (n >> 3), ull(num_unary(I.op, uint32_t(ap))));
+        o1 = mkport(T_OP, NT_SYM, n);
+      } else if (era) {
+        o1 = o2 = P_ERA;
+      }
+    } else {  // I_OPNUM: operator and right operand in the instruction; I_OPRED: number and operator in B
+      const bool red = kind == I_OPRED;
+      const uint32_t op = red ? uint32_t(B >> 32) : I.op;
+      if (num) {
+        x.oper++;
+        o2 = red ? binary_op(c.net, uint32_t(B), op, uint32_t(ap)) : binary_op(c.net, uint32_t(ap), op, uint32_t(I.port));
+      } else if (era) {
+        o2 = P_ERA;
+      } else {
+        bp = mkport(T_OP, red ? unsigned(NT_SYM) : op, n);
+        st_gpu(g_P.heap + (n >> 3), red ? ull(num_unary(op, uint32_t(B))) : ull(uint32_t(I.port)));
+      }
+    }
+    if (kind < I_OPNUM || kind == I_SWITCH) R[I.b * S] = o1;
+    R[I.c * S] = o2;
+  }
+  const bool alast = (I.d & INS_A_LAST) != 0, blast = (I.d & INS_B_LAST) != 0;
+  // link
+  const bool both = principal(ap) && principal(bp);
+  const bool acas = link && aw && !both && ptag(ap) == T_VAR, bcas = link && bw && !both && ptag(bp) == T_VAR;
+  ull ra = pvar(A), rb = pvar(B);
+  if (acas) ra = atom_cas(heap_at(c.net, paddr(ap)), pvar(A), bp);
+  if (bcas) rb = atom_cas(heap_at(c.net, paddr(bp)), pvar(B), ap);
+  if (link) {
+    if (both) {
+      if (skippable(ap) && skippable(bp)) x.eras++;
+      else push(c, ap, bp);
+    } else {
+      // ports that are not behind wires name words of nodes this lane made
+      if (!aw && ptag(ap) == T_VAR) st_gpu(g_P.heap + (paddr(ap) >> 3), bp);
+      if (!bw && ptag(bp) == T_VAR) st_gpu(g_P.heap + (paddr(bp) >> 3), ap);
+    }
+  }
+  if (aw) {
+    if (ra == pvar(A)) wire_done(c, x, A, alast);
+    else wire_failed(c, ap, A, bp, x.nf++, alast);
+  }
+  if (bw) {
+    if (rb == pvar(B)) wire_done(c, x, B, blast);
+    else wire_failed(c, bp, B, ap, x.nf++, blast);
+  }
+}
+// The counters of an interaction that ran instructions.
+HVM_INL void exec_counts(const Ctx c, const Exec& x, bool def, unsigned links) {
+  if (x.anni) count(c, RW_ANNI, x.anni);
+  if (x.oper) count(c, RW_OPER, x.oper);
+  if (x.eras) count(c, RW_ERAS, x.eras);
+  if (def) {
+    count(c, EX_DNODES, x.nodes);
+    count(c, EX_DLINKS, links);
+  }
+}
+template <unsigned S> HVM_INL void exec_def(const Ctx c, const DevDef& d, ull t0, ull* R) {
+  Exec x;
+  R[0] = t0;
+  const DevInstr* ins = g_P.instrs + d.ins_off;
+  for (unsigned k = 0; k < d.ins_len; k++) exec_ins<S>(c, x, ins[k], R);
+  exec_counts(c, x, true, d.links);
+}
+// A Def call outside a step's shared instruction stream, or one that needs
+// more registers than the warp's shared memory holds for a lane.
+HVM_COLD void exec_large(const Ctx c, const DevDef& d, ull t0) {
   if (d.nregs <= LOCAL_REGS) {
     ull R[LOCAL_REGS];
-    return exec(c, d, t0, R, 1, g_P.instrs + d.ins_off);
+    return exec_def<1>(c, d, t0, R);
   }
   // (the reference grows its register scratch to any Def, runtime/src/def.rs:221-223)
   if (!c.W->bigregs || d.nregs > MAX_REGS) return run_fail(c.net, HVM64_ERR_BAD_INPUT, d.nregs);
-  exec(c, d, t0, c.W->bigregs + c.lane, 32, g_P.instrs + d.ins_off);
+  exec_def<32>(c, d, t0, c.W->bigregs + c.lane);
 }
 // A compiled build (hvm64 compile) includes the Book's Defs as functions;
 // they run when the loaded Book is the one they were generated from.
 #ifdef HVM_GEN_INCLUDE
 #include HVM_GEN_INCLUDE
+HVM_COLD bool gen_run(const Ctx c, unsigned id, ull t0) {
+  unsigned before = LS(allocs);
+  bool done = gen_call(c, id, t0);
+  count(c, EX_DNODES, LS(allocs) - before);
+  return done;
+}
 #endif
-HVM_COLD void run_def(const Ctx& c, unsigned id, ull t0) {
-  PROF_RULE(5)
+HVM_COLD void run_def(const Ctx c, unsigned id, ull t0) {
   if (id >= g_P.ndefs) return run_fail(c.net, HVM64_ERR_BAD_INPUT, id);
 #ifdef HVM_GEN_INCLUDE
-  if (g_P.gen && gen_call(c, id, t0)) return;
+  if (g_P.gen && gen_run(c, id, t0)) return;
 #endif
-  ull* R = c.W->regs + c.lane;
-  if (id == c.W->icache_def) {  // staged by the warp for this step
-    const DevDef& d = c.W->idef;
-    if (d.nregs <= SMALL_REGS) return exec(c, d, t0, R, 32, c.W->icache);
-    return exec_large(c, d, t0);
-  }
   const DevDef d = g_P.defs[id];
-  if (d.nregs <= SMALL_REGS) exec(c, d, t0, R, 32, g_P.instrs + d.ins_off);
-  else exec_large(c, d, t0);
+  exec_large(c, d, t0);
 }
 
 // def.rs:30-37 (LabSet::has); the expansion agent's set is LabSet::ALL.
-HVM_INL bool def_has(const Ctx& c, ull ref, unsigned lab) {
+HVM_INL bool def_has(const Ctx c, ull ref, unsigned lab) {
   if (ref & X_BIT) return lab < 0xFFFF;
   unsigned id = unsigned((paddr(ref) >> 3) - 1);
   if (id >= g_P.ndefs) {
@@ -1132,13 +1272,13 @@ HVM_INL bool def_has(const Ctx& c, ull ref, unsigned lab) {
 // ---- expansion agent (runtime/src/net.rs:63-108) ----------------------------
 // An agent is a Ref port with X_BIT whose address names a heap word holding
 // its output port (the reference boxes an `ExpandDef { out }`).
-HVM_COLD ull new_expand(const Ctx& c, ull out) {
+HVM_COLD ull new_expand(const Ctx c, ull out) {
   ull w = alloc(c);
   half_free(c, w ^ 8);
   hstore(c, w, out);
   return mkport(T_REF, 0xFFFF, X_BIT | w);
 }
-HVM_COLD ull take_expand(const Ctx& c, ull port) {
+HVM_COLD ull take_expand(const Ctx c, ull port) {
   ull w = paddr(port) & ~X_BIT;
   unsigned it = 0;
   ull out;
@@ -1147,14 +1287,16 @@ HVM_COLD ull take_expand(const Ctx& c, ull port) {
   half_free(c, w);
   return out;
 }
-HVM_COLD void call(const Ctx& c, ull port, ull trg);
-HVM_COLD void expand_call(const Ctx& c, ull self, ull port) {
+HVM_COLD void expand_call(const Ctx c, ull self, ull port) {
   if (ptag(port) == T_REF && port != P_ERA) {
     if (port & X_BIT) {
       ull a = take_expand(c, self), b = take_expand(c, port);
       return link_port_port(c, a, b);
     }
-    return call(c, port, self);
+    // (what call() does for a nilary argument; calling it would make the
+    // call graph recursive, and its stack depth unknown to the compiler)
+    count(c, RW_DREF);
+    return run_def(c, unsigned((paddr(port) >> 3) - 1), self);
   }
   ull out = take_expand(c, self);
   unsigned t = ptag(port);
@@ -1167,49 +1309,138 @@ HVM_COLD void expand_call(const Ctx& c, ull self, ull port) {
   link_wire_port(c, o1 ^ 8, new_expand(c, pvar(n ^ 8)));
 }
 // net.rs:65-69
-HVM_COLD ull expand(const Ctx& c, ull root) {
+HVM_COLD ull expand(const Ctx c, ull root) {
   ull a = alloc(c);
   half_free(c, a ^ 8);
   link_wire_port(c, root, new_expand(c, pvar(a)));
   return a;
 }
 // def.rs:177-189
-HVM_COLD void call(const Ctx& c, ull port, ull trg) {
+HVM_COLD void call(const Ctx c, ull port, ull trg) {
   if (ptag(trg) == T_CTR && !def_has(c, port, plab(trg))) return comm02(c, port, trg);
   count(c, RW_DREF);
   if (port & X_BIT) return expand_call(c, port, trg);
-  unsigned before = LS(allocs);
   run_def(c, unsigned((paddr(port) >> 3) - 1), trg);
-  count(c, EX_DNODES, LS(allocs) - before);
 }
 
 // ---- interact.rs:6-44 ----------------------------------------------------------
-HVM_COLD void interact(const Ctx& c, ull a, ull b) {
-  PROF_RULE(7)
+// The pairs no instruction list covers: a nilary pair, a call whose argument
+// is nilary, the expansion agent, and pairs without a rule.
+HVM_COLD void interact_other(const Ctx c, ull a, ull b) {
   unsigned at = ptag(a), bt = ptag(b);
   if (at <= T_VAR || bt <= T_VAR) return run_fail(c.net, HVM64_ERR_BAD_PAIR, a);
   bool an = at == T_REF || at == T_NUM, bn = bt == T_REF || bt == T_NUM;
   if (at == T_REF && bn && !skippable(a)) return call(c, a, b);
   if (an && bt == T_REF && !skippable(b)) return call(c, b, a);
   if (an && bn) return count(c, RW_ERAS);
-  if (at == T_CTR && bt == T_SWITCH && plab(a) != 0) return comm22(c, a, b);
-  if (at == T_SWITCH && bt == T_CTR && plab(b) != 0) return comm22(c, a, b);
-  if ((at == T_CTR && bt == T_OP) || (at == T_OP && bt == T_CTR)) return comm22(c, a, b);
-  if (at == T_CTR && bt == T_CTR && plab(a) != plab(b)) return comm22(c, a, b);
-  if (at == bt && at >= T_OP) return anni2(c, a, b);
   if (at == T_REF && bt == T_CTR && plab(b) >= plab(a)) return comm02(c, a, b);
-  if (at == T_CTR && bt == T_REF && plab(a) >= plab(b)) return comm02(c, b, a);
-  if (at == T_NUM && bt == T_CTR) return comm02(c, a, b);
-  if (at == T_CTR && bt == T_NUM) return comm02(c, b, a);
-  if (at == T_REF && a == P_ERA) return comm02(c, a, b);
-  if (bt == T_REF && b == P_ERA) return comm02(c, b, a);
+  if (bt == T_REF && at == T_CTR && plab(a) >= plab(b)) return comm02(c, b, a);
   if (at == T_REF) return call(c, a, b);
   if (bt == T_REF) return call(c, b, a);
-  if (at == T_OP && bt == T_NUM) return op_num(c, a, b);
-  if (at == T_NUM && bt == T_OP) return op_num(c, b, a);
-  if (at == T_SWITCH && bt == T_NUM) return switch_num(c, a, b);
-  if (at == T_NUM && bt == T_SWITCH) return switch_num(c, b, a);
   run_fail(c.net, HVM64_ERR_BAD_PAIR, a);
+}
+
+// Sets up registers R[i * S] for redex (a, b) and counts its rule.  Returns the
+// RULES list to run (offset | length << 8), or one of these.
+enum : unsigned { RUN_DEF = 1u << 16, RUN_OTHER = 2u << 16 };
+template <unsigned S> HVM_INL unsigned classify(const Ctx c, Exec& x, ull a, ull b, ull* R, unsigned& id) {
+  // by tag: Ref < Num < Op < Switch < Ctr
+  if (ptag(a) > ptag(b)) {
+    ull t = a;
+    a = b;
+    b = t;
+  }
+  const unsigned at = ptag(a), bt = ptag(b);
+  // nilary pairs, pairs without a rule, expansion agents
+  if (bt <= T_NUM || at <= T_VAR || at == 4 || (at == T_OP && bt == T_SWITCH) ||
+      (at == T_SWITCH && bt == T_CTR && plab(b) == 0) || is_expand(a))
+    return RUN_OTHER;
+  ull b1 = paddr(b);
+  if (b1 >= g_P.heap_bytes) {
+    run_fail_here(HVM64_ERR_BAD_ADDR);
+    b1 = 0;
+  }
+  if (at == T_REF && a != P_ERA) {  // def.rs:177-189
+    if (bt != T_CTR || (plab(b) < plab(a) && def_has(c, a, plab(b)))) {
+      id = unsigned((paddr(a) >> 3) - 1);
+      count(c, RW_DREF);
+      R[0] = b;
+      return RUN_DEF;
+    }
+  }
+  R[0] = b1;
+  R[S] = b1 ^ 8;
+  if (at == T_REF || (at == T_NUM && bt == T_CTR)) {  // comm02, interact.rs:162-168
+    count(c, RW_COMM);
+    R[2 * S] = R[3 * S] = a;
+    return RULE_LINK2 | RULE_LINK2_LEN << 8;
+  }
+  if (at == T_NUM) {
+    if (bt == T_OP) {  // op_num, interact.rs:251-270
+      R[2 * S] = ull(uint32_t(a)) | ull(plab(b)) << 32;
+      return RULE_OP | RULE_OP_LEN << 8;
+    }
+    // switch_num, interact.rs:201-223
+    x.oper++;
+    const uint32_t num = uint32_t(a);
+    const uint32_t n = num_tag(num) == NT_U24 ? num_payload(num) : 0;
+    ull y = alloc_cold(c);
+    R[2 * S] = mkport(T_CTR, 0, y);
+    if (n == 0) {
+      st_gpu(g_P.heap + ((y ^ 8) >> 3), P_ERA);
+      R[3 * S] = pvar(y);
+    } else {
+      ull z = alloc_cold(c);
+      st_gpu(g_P.heap + (y >> 3), P_ERA);
+      st_gpu(g_P.heap + ((y ^ 8) >> 3), mkport(T_CTR, 0, z));
+      st_gpu(g_P.heap + (z >> 3), ull(num_u24(n - 1)));
+      R[3 * S] = pvar(z ^ 8);
+    }
+    return RULE_LINK2 | RULE_LINK2_LEN << 8;
+  }
+  ull a1 = paddr(a);
+  if (a1 >= g_P.heap_bytes) {
+    run_fail_here(HVM64_ERR_BAD_ADDR);
+    a1 = 0;
+  }
+  R[2 * S] = a1;
+  R[3 * S] = a1 ^ 8;
+  if (at == bt && (at != T_CTR || plab(a) == plab(b))) {  // anni2, interact.rs:72-79
+    x.anni++;
+    return RULE_LINK2 | RULE_LINK2_LEN << 8;
+  }
+  // comm22, interact.rs:118-141
+  count(c, RW_COMM);
+  count(c, EX_COMM22);
+  ull n[4];
+  for (int k = 0; k < 4; k++) n[k] = alloc_cold(c);  // two copies of a, two of b
+  st_gpu(g_P.heap + (n[0] >> 3), pvar(n[2]));
+  st_gpu(g_P.heap + (n[2] >> 3), pvar(n[0]));
+  st_gpu(g_P.heap + ((n[0] ^ 8) >> 3), pvar(n[3]));
+  st_gpu(g_P.heap + (n[3] >> 3), pvar(n[0] ^ 8));
+  st_gpu(g_P.heap + (n[1] >> 3), pvar(n[2] ^ 8));
+  st_gpu(g_P.heap + ((n[2] ^ 8) >> 3), pvar(n[1]));
+  st_gpu(g_P.heap + ((n[1] ^ 8) >> 3), pvar(n[3] ^ 8));
+  st_gpu(g_P.heap + ((n[3] ^ 8) >> 3), pvar(n[1] ^ 8));
+  // b's wires get copies of a, a's wires copies of b
+  R[4 * S] = mkport(at, plab(a), n[0]);
+  R[5 * S] = mkport(at, plab(a), n[1]);
+  R[6 * S] = mkport(bt, plab(b), n[2]);
+  R[7 * S] = mkport(bt, plab(b), n[3]);
+  return RULE_LINK4 | RULE_LINK4_LEN << 8;
+}
+static_assert(SMALL_REGS >= 8, "comm22's registers");
+
+// One interaction of one lane (the reducer's warps run the same steps with
+// their instructions staged, see reduce_kernel).
+HVM_COLD void interact(const Ctx c, ull a, ull b) {
+  Exec x;
+  ull* R = c.W->regs + c.lane;
+  unsigned id = 0, p = classify<32>(c, x, a, b, R, id);
+  if (p == RUN_OTHER) return interact_other(c, a, b);
+  if (p == RUN_DEF) return run_def(c, id, R[0]);
+  for (unsigned k = 0; k < p >> 8; k++) exec_ins<32>(c, x, RULES[(p & 0xFF) + k], R);
+  exec_counts(c, x, false, 0);
 }
 
 // ---- normal-form gather (device-side readback) -------------------------------

@@ -477,6 +477,7 @@ struct RawInstr {
   uint16_t lab = 0;
   uint32_t a = 0, b = 0, c = 0, d = 0;
   uint64_t port = 0;
+  uint8_t flags = 0;  // INS_A_LAST | INS_B_LAST
 };
 
 struct Encoder {
@@ -615,9 +616,16 @@ static uint32_t rename(std::vector<RawInstr>& ins, uint32_t ntrgs) {
   std::vector<uint32_t> freelist;
   uint32_t nregs = 1;
   reg[0] = 0;
-  auto use = [&](uint32_t& t) {
+  // Wire pairs: a TrgId's partner, and whether the TrgId was read already.
+  std::vector<uint32_t> partner(ntrgs, ~0u);
+  auto pair = [&](uint32_t t, uint32_t u) {
+    partner[t] = u;
+    partner[u] = t;
+  };
+  auto use = [&](uint32_t& t, uint8_t& flags, uint8_t last) {
     if (t >= ntrgs || reg[t] < 0) throw Error(HVM64_ERR_BAD_INPUT, "internal: trg read before write");
     uint32_t r = uint32_t(reg[t]);
+    if (partner[t] == t || (partner[t] != ~0u && reg[partner[t]] == -2)) flags |= last;
     reg[t] = -2;
     freelist.push_back(r);
     t = r;
@@ -632,11 +640,26 @@ static uint32_t rename(std::vector<RawInstr>& ins, uint32_t ntrgs) {
   for (RawInstr& i : ins) {
     switch (i.k) {
       case I_CONST: def(i.a); break;
-      case I_LINK: use(i.a); use(i.b); break;
-      case I_LINKCONST: use(i.a); break;
-      case I_CTR: case I_OP: case I_SWITCH: use(i.a); def(i.b); def(i.c); break;
-      case I_OPNUM: use(i.a); def(i.c); break;
-      case I_WIRES: def(i.a); def(i.b); def(i.c); def(i.d); break;
+      case I_LINK:
+        use(i.a, i.flags, INS_A_LAST);
+        use(i.b, i.flags, INS_B_LAST);
+        break;
+      case I_LINKCONST: use(i.a, i.flags, INS_A_LAST); break;
+      case I_CTR: case I_OP: case I_SWITCH:
+        use(i.a, i.flags, INS_A_LAST);
+        if (i.k == I_CTR) pair(i.b, i.c);
+        if (i.k == I_SWITCH) pair(i.c, i.c);  // a wire whose node's other word is free
+        def(i.b);
+        def(i.c);
+        break;
+      case I_OPNUM: use(i.a, i.flags, INS_A_LAST); def(i.c); break;
+      case I_WIRES:
+        pair(i.b, i.d);
+        def(i.a);
+        def(i.b);
+        def(i.c);
+        def(i.d);
+        break;
     }
   }
   return nregs;
@@ -655,7 +678,8 @@ static void emit(Book& book, const std::vector<RawInstr>& raw, uint32_t nregs, D
     x.k = r.k;
     x.op = r.op;
     x.lab = r.lab;
-    x.a = uint8_t(r.a); x.b = uint8_t(r.b); x.c = uint8_t(r.c); x.d = uint8_t(r.d);
+    x.a = uint8_t(r.a); x.b = uint8_t(r.b); x.c = uint8_t(r.c);
+    x.d = r.k == I_WIRES ? uint8_t(r.d) : r.flags;
     x.port = r.port;
     book.instrs.push_back(x);
     nodes += r.k == I_SWITCH ? 3 : (r.k == I_CTR || r.k == I_OP || r.k == I_OPNUM || r.k == I_WIRES) ? 1 : 0;
@@ -663,6 +687,7 @@ static void emit(Book& book, const std::vector<RawInstr>& raw, uint32_t nregs, D
   }
   d.nodes = nodes;
   d.redexes = links + nodes;
+  d.links = links;
 }
 }  // namespace
 
@@ -959,7 +984,7 @@ std::string compile_defs_cuda(const Book& book) {
     if (d.ins_len > MAX_INS || (n > ALL_BELOW && roots_reaching[id] < 2)) continue;
     done.push_back(id);
     o += "// @" + book.names[id] + "\n";
-    o += "HVM_COLD void gen_def_" + std::to_string(id) + "(const Ctx& c, ull r0) {\n";
+    o += "HVM_COLD void gen_def_" + std::to_string(id) + "(const Ctx c, ull r0) {\n";
     if (d.nregs > 1) {
       o += "  ull";
       for (uint32_t k = 1; k < d.nregs; k++) o += (k > 1 ? ", " : " ") + r(k);
@@ -992,7 +1017,7 @@ std::string compile_defs_cuda(const Book& book) {
     o += "}\n";
   }
   o += "\n// The Def's function for Def `id` (false: none; the VM runs it).\n";
-  o += "HVM_INL bool gen_call(const Ctx& c, unsigned id, ull t0) {\n  switch (id) {\n";
+  o += "HVM_INL bool gen_call(const Ctx c, unsigned id, ull t0) {\n  switch (id) {\n";
   for (uint32_t id : done)
     o += "    case " + std::to_string(id) + "u: gen_def_" + std::to_string(id) + "(c, t0); return true;\n";
   o += "  }\n  return false;\n}\n";

@@ -47,11 +47,16 @@ struct DevInstr {  // 16 bytes
   uint8_t k;
   uint8_t op;    // NumTag for Op / OpNum
   uint16_t lab;  // Ctr label
-  uint8_t a, b, c, d;  // registers
+  uint8_t a, b, c, d;  // registers (Wires); d holds INS_* flags in the others
   uint64_t port;  // Const / LinkConst port, OpNum right operand (low 32 bits)
 };
 
-struct DevDef {  // 32 bytes
+// Register a (b) may hold the later consumed one of a node's two wires: a
+// constructor's two results, and the two wires an I_WIRES makes, are pairs; a
+// switch's result is a wire by itself.
+constexpr uint8_t INS_A_LAST = 1, INS_B_LAST = 2;
+
+struct DevDef {  // 36 bytes
   uint32_t ins_off, ins_len;
   uint32_t nregs;
   uint32_t lab_off, lab_len;  // label bitset words in the shared table
@@ -59,11 +64,12 @@ struct DevDef {  // 32 bytes
   uint16_t flags;  // DEF_EXPR | DEF_INERT
   uint32_t nodes;  // upper bound on nodes one call allocates
   uint32_t redexes;
+  uint32_t links;  // I_LINK and I_LINKCONST instructions
 };
 constexpr uint16_t DEF_EXPR = 1;   // an expression program: booting it counts no DREF
 constexpr uint16_t DEF_INERT = 2;  // an inert Def (pre-reduce): its body is one I_CAPTURE
 static_assert(sizeof(DevInstr) == 16, "DevInstr layout");
-static_assert(sizeof(DevDef) == 32, "DevDef layout");
+static_assert(sizeof(DevDef) == 36, "DevDef layout");
 
 // A Def call's registers: up to LOCAL_REGS in the calling thread's local
 // memory; more (up to MAX_REGS, the reach of a DevInstr's one-byte register

@@ -332,7 +332,7 @@ __device__ __noinline__ void serve_complete(WarpSmem& W, unsigned slot) {
 // Take the next request, if the host has written one, and boot it in this
 // warp: its first redexes land in the (empty) ring.  Lane 0 only; returns the
 // slot + 1, or 0.
-__device__ __noinline__ unsigned serve_admit(WarpSmem& W, Ctx& c) {
+__device__ __noinline__ unsigned serve_admit(WarpSmem& W, Ctx c) {
   Ctrl* C = g_P.ctrl;
   ull t = ld_gpu(&C->req_tail);
   ull h = ld_gpu(&C->req_head);
@@ -400,9 +400,7 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
   Ctx c{&W, lane, 0};
   lane_init(&W, lane);
   if (lane < unsigned(NCOUNT)) W.rw[lane] = 0;
-#ifdef HVM_PROFILE_OPS
-  W.prof[lane] = 0;
-#endif
+  if (lane < RULE_INS) W.rules[lane] = RULES[lane];
   if (lane == 0) {
     W.pool_n = 0;
     W.freed_n = 0;
@@ -416,7 +414,7 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     W.bigregs = g_P.bigregs ? g_P.bigregs + ull(32 * MAX_REGS) * gw : nullptr;
     W.sp_cap = g_P.spill ? g_P.spill_cap : 0u;
     W.sp_n = 0;
-    W.st_steps = W.st_lanes = W.st_busy = W.st_idle = W.st_lane_sum = W.st_lane_max = 0;
+    W.st_steps = W.st_lanes = W.st_busy = W.st_idle = 0;
   }
   __syncwarp();
   unsigned top = 0, bot = 0;  // warp-uniform ring indices
@@ -425,7 +423,6 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
   unsigned idle = 0, step = 0;
   // Deadline from this launch's start (a replayed launch gets a fresh one).
   const ull deadline = globaltimer() + C->timeout_ns;
-  const long long born = clock64();
   unsigned nap = 0;  // idle backoff, ns
 
   for (;;) {
@@ -461,8 +458,9 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       if (cur >= 0) {
         flush_counters(W, cur);
         int fin = 0;
+        if (g_P.serve) __threadfence();  // this warp's heap writes, before its share is released
+        __syncwarp();
         if (lane == 0) {
-          if (g_P.serve) __threadfence();  // this warp's heap writes, before its share is released
           long long old = (long long)atomicAdd(reinterpret_cast<ull*>(&g_P.nets[cur].pending), ~0ull);
           fin = old == 1;
           if (fin && g_P.serve) serve_complete(W, unsigned(cur));
@@ -644,8 +642,8 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
 #pragma unroll
     for (int q = QW - 1; q >= 0; q--) {
       if (st[q]) {
-        W.sel[2 * sr[q]] = qa[q];
-        W.sel[2 * sr[q] + 1] = qb[q];
+        W.regs[2 * sr[q]] = qa[q];  // (the registers are free between steps)
+        W.regs[2 * sr[q] + 1] = qb[q];
       }
       if (su[q]) {
         unsigned k = (base + below + unsigned(__popc(um[q] & gt))) & (SCAP - 1);
@@ -659,8 +657,8 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       __syncwarp();
       if (lane >= n && lane < nsel32) {
         unsigned k = (top + lane - n) & (SCAP - 1);
-        S[2 * k] = W.sel[2 * lane];
-        S[2 * k + 1] = W.sel[2 * lane + 1];
+        S[2 * k] = W.regs[2 * lane];
+        S[2 * k + 1] = W.regs[2 * lane + 1];
       }
       top += nsel32 - n;
     }
@@ -669,56 +667,90 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       W.ring_base = top;
       W.ring_cap = unsigned(SCAP) - (top - bot);
     }
-    // A step of Def calls: stage that Def's instructions in shared memory
-    // (one cooperative load instead of a dependent fetch per instruction).
+    // A step of Def calls: stage that Def's header and first ICACHE
+    // instructions in shared memory (one cooperative load instead of a
+    // dependent fetch per instruction).
     // Every lane reads the staged Def's index before lane 0 may replace it:
     // lanes are not guaranteed to run this in lock-step, and a lane that saw
     // the new index would skip its share of the copy.
     __syncwarp();
     const unsigned staged = W.icache_def;
+    ull ra = 0, rb = 0;
+    if (lane < n) {
+      ra = W.regs[2 * lane];
+      rb = W.regs[2 * lane + 1];
+    }
     __syncwarp();
-#ifdef HVM_GEN_INCLUDE
-    const bool vm_def = !(g_P.gen && key - 64u < HVM_GEN_NDEFS);  // compiled Defs need no staging
-#else
-    const bool vm_def = true;
-#endif
-    if (key >= 64u && key - 64u < g_P.ndefs && key - 64u != staged && vm_def) {
-      unsigned id = key - 64u;
-      const DevDef d = g_P.defs[id];
-      if (d.ins_len <= ICACHE) {
-        const uint4* src = reinterpret_cast<const uint4*>(g_P.instrs + d.ins_off);
-        uint4* dst = reinterpret_cast<uint4*>(W.icache);
-        for (unsigned i = lane; i < d.ins_len; i += 32) dst[i] = __ldg(src + i);
-        if (lane == 0) {
-          W.idef = d;
-          W.icache_def = id;
-        }
-      } else if (lane == 0) {
-        W.icache_def = ~0u;
+    const bool is_def = key >= 64u && key - 64u < g_P.ndefs;
+    if (is_def && key - 64u != staged) {
+      const DevDef d = g_P.defs[key - 64u];
+      const uint4* src = reinterpret_cast<const uint4*>(g_P.instrs + d.ins_off);
+      if (lane < min(d.ins_len, ICACHE)) reinterpret_cast<uint4*>(W.icache)[lane] = __ldg(src + lane);
+      if (lane == 0) {
+        W.idef = d;
+        W.icache_def = key - 64u;
       }
     }
     long long s0c = clock64();
     __syncwarp();
-    unsigned mine = 0;
-    if (lane < n) {
-      long long l0 = clock64();
-      interact(c, W.sel[2 * lane], W.sel[2 * lane + 1]);
-      // (a call to settle only when the lane freed a word alone: measured
-      // 5 % faster than calling it to find out)
-      if (W.fw[lane] | W.fw[32 + lane] | W.fw[64 + lane] | W.fw[96 + lane]) settle(c);
-      mine = unsigned(min(clock64() - l0, 0x7fffffffll));
+    // Run the redexes: each lane's rule becomes a list of instructions (the
+    // Def's, staged, or one of the rules' own) on its shared-memory registers.
+    {
+      const unsigned dlen = is_def ? W.idef.ins_len : 0u;
+      ull* R = W.regs + lane;
+      const DevInstr* ins = W.rules;
+      unsigned len = 0, id = 0;
+      bool def = false, other = false;
+      Exec x;
+      if (lane < n) {
+        const unsigned p = classify<32>(c, x, ra, rb, R, id);
+        if (p == RUN_DEF) {
+          ins = W.icache;
+          len = dlen;
+          def = true;
+          if (!is_def || W.idef.nregs > SMALL_REGS) {
+            run_def(c, id, R[0]);
+            def = false;
+            other = true;
+            len = 0;
+          }
+#ifdef HVM_GEN_INCLUDE
+          else if (g_P.gen && gen_run(c, id, R[0])) {
+            def = false;
+            other = true;
+            len = 0;
+          }
+#endif
+        } else if (p == RUN_OTHER) {
+          interact_other(c, ra, rb);
+          other = true;
+        } else {
+          ins = W.rules + (p & 0xFFu);
+          len = p >> 8;
+        }
+      }
+      for (unsigned base = 0;;) {
+        const unsigned end = min(len, base + ICACHE);
+        for (unsigned k = base; k < end; k++) exec_ins<32>(c, x, ins[k - base], R);
+        base += ICACHE;
+        if (base >= dlen) break;
+        // (a Def longer than the staged window: load the next one)
+        __syncwarp();
+        const uint4* src = reinterpret_cast<const uint4*>(g_P.instrs + W.idef.ins_off + base);
+        if (lane < min(dlen - base, ICACHE)) reinterpret_cast<uint4*>(W.icache)[lane] = __ldg(src + lane);
+        if (lane == 0) W.icache_def = ~0u;
+        __syncwarp();
+      }
+      if (lane < n) {
+        exec_counts(c, x, def, W.idef.links);
+        if ((other || x.nf) && (W.fw[lane] | W.fw[32 + lane])) settle(c);
+      }
     }
     __syncwarp();
-    {
-      unsigned mx = __reduce_max_sync(0xffffffffu, mine);
-      unsigned sm = __reduce_add_sync(0xffffffffu, mine);
-      if (lane == 0) {
-        W.st_busy += ull(clock64() - s0c);
-        W.st_lanes += n;
-        W.st_steps++;
-        W.st_lane_sum += sm;
-        W.st_lane_max += mx;
-      }
+    if (lane == 0) {
+      W.st_busy += ull(clock64() - s0c);
+      W.st_lanes += n;
+      W.st_steps++;
     }
     {
       const unsigned cnt = W.ring_cnt;
@@ -732,9 +764,8 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     // folding every step measured 4 % slower.
     if ((step & 4095) == 0) fold_counts_cold(W, cur);
     else __syncwarp();
-    // Nodes reclaimed in this step become allocatable after a fence.
-    mem_fence();
-    __syncwarp();
+    // Nodes reclaimed in this step become allocatable.  (No fence: their words
+    // hold LOCK by completed exchanges, or the lane that stored it fenced.)
     {
       int pn = max(W.pool_n, 0);
       int fn = min(W.freed_n, POOL);
@@ -788,12 +819,6 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     atomicAdd(&C->stat_lanes, W.st_lanes);
     atomicAdd(&C->stat_busy_cycles, W.st_busy);
     atomicAdd(&C->stat_idle_cycles, W.st_idle);
-    atomicAdd(&C->stat_lane_sum, W.st_lane_sum);
-    atomicAdd(&C->stat_lane_max, W.st_lane_max);
-    atomicAdd(&C->stat_total, ull(clock64() - born));
-#ifdef HVM_PROFILE_OPS
-    for (int k = 0; k < 32; k++) atomicAdd(&C->stat_prof[k], W.prof[k]);
-#endif
   }
 }
 
@@ -1216,8 +1241,6 @@ struct Runner {
 
     stat_donated = stat_spilled = stat_overflow = 0;
     stat_steps = stat_lanes = stat_busy = stat_idle = 0;
-    for (int k = 0; k < 8; k++) stat_g_steps[k] = stat_g_cycles[k] = 0;
-    for (int k = 0; k < 32; k++) stat_prof[k] = 0;
     cudaStream_t st = 0;
     cudaEvent_t e0, e1;
     CU(cudaEventCreate(&e0));
@@ -1253,10 +1276,6 @@ struct Runner {
       stat_lanes += host_ctrl.stat_lanes;
       stat_busy += host_ctrl.stat_busy_cycles;
       stat_idle += host_ctrl.stat_idle_cycles;
-      for (int k = 0; k < 32; k++) stat_prof[k] += host_ctrl.stat_prof[k];
-      stat_g_steps[0] += host_ctrl.stat_lane_sum;
-      stat_g_steps[1] += host_ctrl.stat_lane_max;
-      stat_g_steps[2] += host_ctrl.stat_total;
       bump = std::min<uint64_t>(host_ctrl.bump, heap_bytes / 16);
       if (host_ctrl.error) {
         for (unsigned k = first; k < first + count; k++) host_nets[k].status = host_ctrl.error;
@@ -1419,7 +1438,6 @@ struct Runner {
 
   uint64_t stat_donated = 0, stat_spilled = 0, stat_overflow = 0, heap_used = 0;
   uint64_t stat_steps = 0, stat_lanes = 0, stat_busy = 0, stat_idle = 0;
-  uint64_t stat_g_steps[8] = {0}, stat_g_cycles[8] = {0}, stat_prof[32] = {0};
 
   void stats(hvm64_stats* o) const {
     *o = hvm64_stats{};
@@ -2038,15 +2056,6 @@ int hvm64_batch_stats(const hvm64_batch* b, hvm64_stats* out) {
   b->r.stats(out);
   return HVM64_OK;
 }
-// Diagnostic (not in the public header): steps and cycles of the last run
-// by the number of distinct rule classes among the lanes of a step.
-int hvm64_internal_class_steps(const hvm64_batch* b, uint64_t* steps8, uint64_t* prof32) {
-  if (!b) return HVM64_ERR_BAD_INPUT;
-  for (int k = 0; k < 8; k++) steps8[k] = b->r.stat_g_steps[k];
-  for (int k = 0; k < 32; k++) prof32[k] = b->r.stat_prof[k];
-  return HVM64_OK;
-}
-
 int hvm64_net_stats(const hvm64_net* n, hvm64_stats* out) {
   if (!n || !out) return hvm::set_error(HVM64_ERR_BAD_INPUT, "null argument");
   n->r.stats(out);
