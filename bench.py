@@ -572,7 +572,7 @@ def main():
         "roofline": roofline_record(alg / K, atoms / K, ksec / K, hbm, peak_kind, arate, anote,
                                     tpi * total_per_rank / K if tpi else None, tcap,
                                     "reduce_kernel (+ boot_kernel) device time per launch (one launch per step)"),
-        "gpu_launches": 4 * K,
+        "gpu_launches": 2 * K,
         "tuning": {"knobs": {key: getattr(tune, key) for key in ("blocks_per_sm", "chunk_nodes", "donate_min",
                                                                   "queue_slots_log2", "max_warps_per_net")},
                    "cuda_graph": True, "autotune": tune_report},

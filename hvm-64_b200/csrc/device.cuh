@@ -73,16 +73,16 @@ struct Ctrl {
   ull deadline;    // %globaltimer ns
   ull donate_min;
   ull max_warps;   // holders (warps + queued slots) per net beyond which no work is donated; 0: no cap
-  ull q_mask;
+  ull q_mask;      // queue capacity - 1
+  ull q_base;      // the run's first ticket
+  ull q_warps;     // reducer warps
   int error;
   int error_net;
   ull error_info;
-  ull pad0[6];
+  ull pad0[4];
   long long nets_left;
-  ull pad1[15];
-  long long hungry;
-  ull pad2[15];
-  ull q_head;
+  ull pad1[31];
+  ull q_head;      // pop tickets taken: ahead of q_tail by the warps that wait
   ull pad3[15];
   ull q_tail;
   ull pad4[15];
@@ -394,7 +394,7 @@ struct alignas(16) WarpSmem {
   ull* bigregs;               // this warp's register files for Defs above LOCAL_REGS (null: none)
   unsigned sp_n, sp_cap;      // redexes in it between steps, and its capacity
   int pool_cap;               // 0: no reuse pool (reclaimed nodes go to `ovf`)
-  ull st_steps, st_lanes, st_busy, st_idle;
+  ull st_steps, st_lanes, st_busy, st_idle, st_donated, st_spilled;
   unsigned ring_cnt;
   int pool_n;
   int freed_n;

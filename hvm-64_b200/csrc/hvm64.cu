@@ -1,14 +1,13 @@
 // Kernels, device queue, runner and C ABI of the B200 interaction-net reducer.
 //
-// Work distribution.  Each warp owns a LIFO redex stack in shared memory and
-// processes up to 32 redexes per step, one per lane.  Redexes an interaction
-// creates collect in a per-lane buffer and are appended to the warp's stack
-// after the step (warp prefix sum).  Work moves between warps through one
-// global lock-free queue of 32-redex slots (bounded MPMC ring with per-slot
-// sequence numbers): a warp whose stack is deep donates its oldest redexes
-// when other warps are hungry, spills when its stack would overflow, and an
-// idle warp takes a slot.  A warp holds one net's work at a time, so batched
-// reduction attributes every interaction to its net without tagging redexes.
+// Work distribution.  Each warp owns a LIFO redex stack in shared memory (and
+// an overflow stack in device memory) and processes up to 32 redexes per
+// step, one per lane, pushing the redexes they create.  Work moves between
+// warps through one global ring of 32-redex slots handed out by tickets: a
+// warp out of work waits at its own slot, and a warp whose step leaves
+// redexes waiting fills slots while others wait.  A warp holds one net's work
+// at a time, so batched reduction attributes every interaction to its net
+// without tagging redexes.
 //
 // Termination, per net: `pending` counts the warps holding the net's work plus
 // the net's queued slots.  A warp that takes a slot inherits the slot's unit;
@@ -35,18 +34,34 @@ namespace hvm {
 namespace dev {
 
 // ---- global redex queue --------------------------------------------------------
-// Single-thread reservation; data movement may be done by the whole warp.
-// Never waits for a consumer: a full queue returns false at once and the
-// caller keeps the work.  A lost CAS means another producer got its slot, so
-// retrying under contention always makes progress; the retry count is still
-// bounded (then the reservation fails like a full queue).
+// A ring of slots handed out by two ticket counters.  A warp out of work takes
+// one pop ticket with a fetch-and-add and then polls that slot's own sequence
+// word until a push fills it, so waiting warps share no line; a push takes its
+// ticket with a fetch-and-add too.  q_head - q_tail is then the number of warps
+// that wait with nothing on its way to them.  (With one CAS loop per end and
+// every idle warp polling the head, the queue moved one slot in 0.8 us however
+// many warps wanted one: a tree sum of 2^18 leaves spent its 18 ms on 23,700
+// slots, and sharing more work made it slower.)
+//
+// Sequence words: `pos` free for ticket pos, pos + 1 filled, pos + capacity
+// emptied (free for the next lap).  A run's tickets start at Ctrl::q_base, a
+// multiple of the capacity above every earlier run's, and a word below the
+// base counts as free for its first lap: no run initialises the ring.
+__device__ __forceinline__ ull q_seq(ull pos) {
+  Ctrl* C = g_P.ctrl;
+  ull s = ld_gpu(&g_P.q[pos & C->q_mask].seq);
+  return s < C->q_base ? C->q_base + (pos & C->q_mask) : s;
+}
+// Single-thread reservation by CAS, for a push that must not wait for
+// anything: a full queue returns false at once and the caller keeps the work.
+// A lost CAS means another push got its slot, so retrying under contention
+// always makes progress; the retry count is still bounded (then the
+// reservation fails like a full queue).
 __device__ bool q_reserve_push(ull& pos) {
   Ctrl* C = g_P.ctrl;
-  ull mask = C->q_mask;
   pos = ld_gpu(&C->q_tail);
   for (unsigned tries = 0; tries < (1u << 20); tries++) {
-    Slot* s = &g_P.q[pos & mask];
-    long long dif = (long long)ld_gpu(&s->seq) - (long long)pos;
+    long long dif = (long long)(q_seq(pos) - pos);
     if (dif == 0) {
       ull old = atomicCAS(&C->q_tail, pos, pos + 1);
       if (old == pos) return true;
@@ -60,28 +75,26 @@ __device__ bool q_reserve_push(ull& pos) {
   }
   return false;
 }
+// Reservation by fetch-and-add (one pushing lane per warp, q_warps warps).
+// The test leaves room for every warp's push and every lane's overflow push
+// (q_reserve_push) that may be between its own test and its ticket, so the
+// slot's previous holder has its pop ticket; at most this waits for that warp
+// to copy the slot out (bounded).  Queues too small for that use the CAS.
+__device__ bool q_ticket_push(unsigned net, ull& pos) {
+  Ctrl* C = g_P.ctrl;
+  long long used = (long long)(ld_gpu(&C->q_tail) - ld_gpu(&C->q_head));
+  if (used + 40 * (long long)C->q_warps > (long long)C->q_mask) return q_reserve_push(pos);
+  pos = atomicAdd(&C->q_tail, 1ull);
+  if (pos - C->q_base > C->q_mask) {  // past the first lap
+    unsigned it = 0;
+    while (q_seq(pos) != pos)
+      if (!run_spin(net, it)) return false;
+  }
+  return true;
+}
 __device__ void q_publish(ull pos) {
   __threadfence();
   st_gpu(&g_P.q[pos & g_P.ctrl->q_mask].seq, pos + 1);
-}
-__device__ bool q_reserve_pop(ull& pos) {
-  Ctrl* C = g_P.ctrl;
-  ull mask = C->q_mask;
-  pos = ld_gpu(&C->q_head);
-  for (int tries = 0; tries < 64; tries++) {
-    Slot* s = &g_P.q[pos & mask];
-    long long dif = (long long)ld_gpu(&s->seq) - (long long)(pos + 1);
-    if (dif == 0) {
-      ull old = atomicCAS(&C->q_head, pos, pos + 1);
-      if (old == pos) return true;
-      pos = old;
-    } else if (dif < 0) {
-      return false;  // empty
-    } else {
-      pos = ld_gpu(&C->q_head);
-    }
-  }
-  return false;
 }
 __device__ void q_release(ull pos) {
   __threadfence();
@@ -117,7 +130,7 @@ __device__ bool donate_vals(ull ra, ull rb, unsigned cnt, int cur) {
   ull pos = 0;
   int ok = 0;
   if (lane == 0) {
-    ok = q_reserve_push(pos) ? 1 : 0;
+    ok = q_ticket_push(unsigned(cur), pos) ? 1 : 0;
     if (ok) atomicAdd(reinterpret_cast<ull*>(&g_P.nets[cur].pending), 1ull);
   }
   ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -129,9 +142,8 @@ __device__ bool donate_vals(ull ra, ull rb, unsigned cnt, int cur) {
     st_gpu(&s->r[2 * lane + 1], rb);
   }
   if (lane == 0) st_gpu(reinterpret_cast<ull*>(&s->net), (ull(cnt) << 32) | unsigned(cur));
-  __threadfence();
   __syncwarp();
-  if (lane == 0) q_publish(pos);
+  if (lane == 0) q_publish(pos);  // (its fence covers the warp's stores before the barrier)
   return true;
 }
 // The `cnt` oldest redexes of the warp's shared-memory stack into a slot.
@@ -366,8 +378,10 @@ __device__ __noinline__ unsigned serve_admit(WarpSmem& W, Ctx c) {
   atomicAdd(reinterpret_cast<ull*>(&C->nets_left), 1ull);
   c.net = slot;
   W.ring_base = 0;
-  W.ring_cap = unsigned(SCAP - HEADROOM);
+  W.ring_cap = SCAP;
   W.ring_cnt = 0;
+  const unsigned sp_cap = W.sp_cap;
+  W.sp_cap = W.sp_n;  // boot redexes past the ring go to the queue
   ull root = alloc(c);
   half_free(c, root ^ 8);  // only the left word is the root wire; the node is reclaimed once it is freed
   if (prog < g_P.ndefs && !(g_P.defs[prog].flags & 1)) W.rw[RW_DREF]++;
@@ -376,9 +390,12 @@ __device__ __noinline__ unsigned serve_admit(WarpSmem& W, Ctx c) {
   root = expand(c, root);
   settle(c);
   st_gpu(&ns.root, root);
+  W.sp_cap = sp_cap;
   return slot + 1;
 }
 
+constexpr unsigned SHARE_PART = 4;  // redexes a shared slot gets at least (1: 5-20 % slower)
+constexpr unsigned POLL_NS = 1000;  // a waiting warp's pause between two looks at its slot
 #ifndef HVM_QW
 #define HVM_QW 2
 #endif
@@ -414,16 +431,17 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     W.bigregs = g_P.bigregs ? g_P.bigregs + ull(32 * MAX_REGS) * gw : nullptr;
     W.sp_cap = g_P.spill ? g_P.spill_cap : 0u;
     W.sp_n = 0;
-    W.st_steps = W.st_lanes = W.st_busy = W.st_idle = 0;
+    W.st_steps = W.st_lanes = W.st_busy = W.st_idle = W.st_donated = W.st_spilled = 0;
   }
   __syncwarp();
   unsigned top = 0, bot = 0;  // warp-uniform ring indices
   int cur = -1;               // the net whose work this warp holds
-  bool hungry = false;
+  bool waiting = false;       // holds a pop ticket
+  ull ticket = 0;
+  unsigned admitted = 0;
   unsigned idle = 0, step = 0;
   // Deadline from this launch's start (a replayed launch gets a fresh one).
   const ull deadline = globaltimer() + C->timeout_ns;
-  unsigned nap = 0;  // idle backoff, ns
 
   for (;;) {
     // The error word is polled only now and then: every warp reading it each
@@ -469,70 +487,62 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
         __syncwarp();
         cur = -1;
       }
-      ull pos = 0;
-      int got = 0;
-      if (lane == 0) got = q_reserve_pop(pos) ? 1 : 0;
-      got = __shfl_sync(0xffffffffu, got, 0);
-      if (!got) {
-        // Idle: back off exponentially (1 us .. 64 us) so that waiting warps
-        // do not crowd the queue's and the counters' L2 lines.
-        int stop = 0;
-        unsigned admitted = 0;
-        if (lane == 0) {
-          if (!hungry) atomicAdd(reinterpret_cast<ull*>(&C->hungry), 1ull);
-          if (g_P.serve) {
-            // Serving: boot the next request here, or end once the host has
-            // asked to stop and nothing is admitted, queued or running.
-            admitted = serve_admit(W, c);
-            if (!admitted && ld_gpu32(&C->stop) && ld_gpu64s(&C->nets_left) <= 0 &&
-                ld_gpu(&C->req_head) >= ld_gpu(&C->req_tail))
-              stop = 1;
-            else if (!admitted && (++idle & 15) == 0 && globaltimer() > deadline) {
-              run_fail(0, HVM64_ERR_TIMEOUT, 3);  // a server lives at most timeout_ms
-              stop = 1;
+      // Wait for a slot: one ticket, polled until it is filled.  Every 8th
+      // poll looks whether the run is over (or, serving, for a request).
+      int got = 0;  // 1: the slot is filled, 2: stop, 3: a request was booted
+      if (lane == 0) {
+        if (!waiting) ticket = atomicAdd(&C->q_head, 1ull);
+        const long long t0 = clock64();
+        for (unsigned polls = 0; !got; polls++) {
+          if (q_seq(ticket) == ticket + 1) {
+            got = 1;
+            break;
+          }
+          if ((polls & 7u) == 7u) {
+            if (g_P.serve) {
+              // Serving: boot the next request here, or end once the host has
+              // asked to stop and nothing is admitted, queued or running.
+              admitted = serve_admit(W, c);
+              if (admitted) got = 3;
+              else if (ld_gpu32(&C->stop) && ld_gpu64s(&C->nets_left) <= 0 && ld_gpu(&C->req_head) >= ld_gpu(&C->req_tail))
+                got = 2;
+            } else if (ld_gpu64s(&C->nets_left) <= 0) {
+              got = 2;
             }
-          } else if (ld_gpu64s(&C->nets_left) <= 0) {
-            stop = 1;
-          } else if ((++idle & 15) == 0 && globaltimer() > deadline) {
-            run_fail(0, HVM64_ERR_TIMEOUT, 1);
-            stop = 1;
+            if (!got && (++idle & 15) == 0 && globaltimer() > deadline) {
+              run_fail(0, HVM64_ERR_TIMEOUT, g_P.serve ? 3 : 1);  // (a server lives at most timeout_ms)
+              got = 2;
+            }
+            if (ld_gpu32(&C->error)) got = 2;
           }
-          if (ld_gpu32(&C->error)) stop = 1;
+          if (!got) __nanosleep(POLL_NS);
         }
-        hungry = true;
-        if (__shfl_sync(0xffffffffu, stop, 0)) break;
+        W.st_idle += ull(clock64() - t0);
+      }
+      waiting = true;
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (got == 2) break;
+      if (got == 3) {
+        // The booted redexes go to the queue, to this warp or another one that
+        // waits; the warp keeps its ticket.
         admitted = __shfl_sync(0xffffffffu, admitted, 0);
-        if (admitted) {
-          if (lane == 0) atomicAdd(reinterpret_cast<ull*>(&C->hungry), ~0ull);
-          hungry = false;
-          nap = 0;
-          idle = 0;
-          cur = int(admitted - 1);
-          c.net = unsigned(cur);
-          bot = 0;
-          __syncwarp();  // lane 0's boot pushes are in shared memory before the others read the count
-          {
-            const unsigned cnt = W.ring_cnt;
-            top = min(cnt, W.ring_cap);
-            const unsigned spilled = spilled_of(&W, cnt);
-            __syncwarp();
-            if (lane == 0) W.sp_n += spilled;
-            __syncwarp();
+        const int net = int(admitted - 1);
+        const unsigned total = min(W.ring_cnt, unsigned(SCAP));
+        __syncwarp();
+        for (unsigned done = 0; done < total; done += unsigned(CHUNK)) {
+          const unsigned k = min(total - done, unsigned(CHUNK));
+          ull ra = lane < k ? S[2 * (done + lane)] : 0, rb = lane < k ? S[2 * (done + lane) + 1] : 0;
+          if (!donate_vals(ra, rb, k, net)) {
+            if (lane == 0) run_fail(unsigned(net), HVM64_ERR_QUEUE, 2);
+            break;
           }
-          continue;
         }
-        // (a serving reducer naps at most 8 us: new requests wait on it)
-        nap = nap ? min(nap * 2, g_P.serve ? 8192u : 65536u) : 1024u;
-        long long t0 = clock64();
-        __nanosleep(nap);
-        if (lane == 0) W.st_idle += ull(clock64() - t0);
+        cur = net;  // released above, like a net whose redexes ran out
         continue;
       }
-      nap = 0;
-      if (hungry && lane == 0) atomicAdd(reinterpret_cast<ull*>(&C->hungry), ~0ull);
-      hungry = false;
+      waiting = false;
       idle = 0;
-      pos = shfl(pos, 0);
+      const ull pos = shfl(ticket, 0);
       __threadfence();
       Slot* s = &g_P.q[pos & C->q_mask];
       unsigned cnt = 0, net = 0;
@@ -586,8 +596,12 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       } else if (!donate(S, bot, 32u, cur)) {
         break;
       }
-      if (lane == 0) atomicAdd(&C->stat_spilled, 1ull);
+      if (lane == 0) W.st_spilled++;
     }
+
+    // (looked at after the selection below: the loads are in flight meanwhile)
+    long long starving = 0;  // warps that wait with nothing on its way
+    if (lane == 0) starving = (long long)(ld_gpu(&C->q_head) - ld_gpu(&C->q_tail));
 
     // Choose this step's redexes: among the newest 32 * QW, the rule class
     // most common among the newest 32 (ties: the newest); up to 32 of that
@@ -661,6 +675,38 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
         S[2 * k + 1] = W.regs[2 * lane + 1];
       }
       top += nsel32 - n;
+    }
+    // Share what this step leaves waiting while other warps starve: the
+    // overflow stack first, then the oldest of the shared-memory stack, in up
+    // to four slots.  A step takes 5-10 us whatever its number of lanes, so
+    // while an eighth of the warps or more starve, any redex that would wait
+    // for the next step is better off in one of them (sort of 2^9 keys: 38.6 ms
+    // sharing from 64 redexes, 20.4 ms from one); when few starve, stacks of
+    // 64 keep the steps full (a batch of 451 nets: 384 ms against 410 ms).
+    // The queue also takes work when the overflow stack is three quarters full.
+    const unsigned left = top - bot + W.sp_n;
+    const bool sp_high = W.sp_n > W.sp_cap - W.sp_cap / 4u;
+    if (left) {
+      int want = 0;
+      if (lane == 0) {
+        const unsigned from = C->donate_min ? unsigned(C->donate_min) : starving * 8 >= (long long)C->q_warps ? 1u : 64u;
+        // a net already spread over max_warps holders (warps and queued
+        // slots) gets no more, except to relieve a full overflow stack
+        const ull cap = C->max_warps;
+        const bool spread = cap && (ull)ld_gpu64s(&g_P.nets[cur].pending) >= cap;
+        want = spread || left < from ? 0 : int(min(max(starving, 0ll), 4ll));
+      }
+      want = __shfl_sync(0xffffffffu, want, 0);
+      unsigned k = 0;
+      for (; k < (sp_high ? 4u : unsigned(want)) && W.sp_n >= 32u; k++) {
+        if (!donate_spill(W, cur)) break;
+        if (lane == 0) W.st_donated++;
+      }
+      for (; k < unsigned(want) && top != bot; k++) {
+        const unsigned parts = unsigned(want) - k, avail = top - bot;
+        if (!donate(S, bot, min(max((avail + parts - 1u) / parts, SHARE_PART), min(avail, 32u)), cur)) break;
+        if (lane == 0) W.st_donated++;
+      }
     }
     if (lane == 0) {
       W.ring_cnt = 0;
@@ -782,36 +828,6 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       }
       __syncwarp();
     }
-
-    // Share work when other warps are starving, and move work to the global
-    // queue when the overflow stack is three quarters full: the overflow
-    // stack first, then the oldest half of the shared-memory stack (at most
-    // four slots per check).
-    const bool sp_high = W.sp_n > W.sp_cap - W.sp_cap / 4u;
-    if (top - bot + W.sp_n >= unsigned(C->donate_min) && ((step & 7) == 0 || sp_high)) {
-      int give = 0;
-      if (lane == 0) {
-        long long h = ld_gpu64s(&C->hungry);
-        long long queued = (long long)(ld_gpu(&C->q_tail) - ld_gpu(&C->q_head));
-        // a net already spread over max_warps holders (warps and queued
-        // slots) gets no more, except to relieve a full overflow stack
-        ull cap = C->max_warps;
-        bool spread = cap && (ull)ld_gpu64s(&g_P.nets[cur].pending) >= cap;
-        give = (h > 0 && queued < h && !spread) ? 2 : sp_high ? 1 : 0;
-      }
-      give = __shfl_sync(0xffffffffu, give, 0);
-      if (give) {
-        unsigned k = 0;
-        for (; k < 4u && W.sp_n >= 32u; k++) {
-          if (!donate_spill(W, cur)) break;
-          if (lane == 0) atomicAdd(&C->stat_donated, 1ull);
-        }
-        for (unsigned chunks = give == 2 ? min((top - bot) / 64u, 4u - k) : 0u; chunks; chunks--) {
-          if (!donate(S, bot, 32u, cur)) break;
-          if (lane == 0) atomicAdd(&C->stat_donated, 1ull);
-        }
-      }
-    }
   }
   if (cur >= 0) flush_counters(W, cur);
   if (lane == 0) {
@@ -819,6 +835,8 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     atomicAdd(&C->stat_lanes, W.st_lanes);
     atomicAdd(&C->stat_busy_cycles, W.st_busy);
     atomicAdd(&C->stat_idle_cycles, W.st_idle);
+    atomicAdd(&C->stat_donated, W.st_donated);
+    atomicAdd(&C->stat_spilled, W.st_spilled);
   }
 }
 
@@ -886,11 +904,19 @@ __global__ void __launch_bounds__(THREADS) boot_kernel(unsigned first, unsigned 
   }
 }
 
-__global__ void set_deadline_kernel(Ctrl* c, ull timeout_ns);
-
-__global__ void queue_init_kernel(Slot* q, ull n) {
+// Sequence words of a new ring: below every run's base.
+__global__ void queue_zero_kernel(Slot* q, ull n) {
   ull i = ull(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) q[i].seq = i;
+  if (i < n) q[i].seq = 0;
+}
+
+// Host side: the queue's part of a run's control block.  `runs` counts the
+// runs that used the queue's buffer (its words were zero before the first).
+constexpr unsigned Q_RUN_BITS = 36;  // tickets one run can hand out: 2^36
+inline void queue_begin(Ctrl& c, unsigned qlog2, unsigned warps, uint64_t& runs) {
+  c.q_mask = (1ull << qlog2) - 1;
+  c.q_warps = warps;
+  c.q_base = c.q_head = c.q_tail = ++runs << Q_RUN_BITS;
 }
 
 }  // namespace dev
@@ -1166,6 +1192,17 @@ struct Runner {
   uint64_t rw_limit = 0;
   DevBuf<dev::ull> capture;
 
+  // The redex queue: zeroed when it is allocated (its sequence words must lie
+  // below every run's q_base), never again.
+  uint64_t queue_runs = 0;
+  void alloc_queue(size_t slots) {
+    if (q.p && q.n >= slots) return;
+    q.alloc(slots);
+    dev::queue_zero_kernel<<<unsigned((slots + 255) / 256), 256>>>(q.p, slots);
+    CU(cudaGetLastError());
+    CU(cudaStreamSynchronize(0));  // (runs may use another stream)
+  }
+
   // The reducer grid for a tuning, and the warps' overflow stacks sized to it.
   DevBuf<dev::ull> spill;
   unsigned spill_cap = 0, grid = 0;
@@ -1191,7 +1228,7 @@ struct Runner {
     CU(cudaGetLastError());
   }
 
-  void reset_ctrl(const hvm64_tuning& t, cudaStream_t st, unsigned qlog2, uint64_t bump) {
+  void reset_ctrl(const hvm64_tuning& t, cudaStream_t st, unsigned qlog2, uint64_t bump, uint64_t timeout_ms) {
     dev::Ctrl c{};
     c.bump = bump;  // node 0 is reserved
     c.heap_nodes = heap_bytes / 16;
@@ -1199,10 +1236,10 @@ struct Runner {
     c.heap_bytes = heap_bytes;
     c.chunk_nodes = t.chunk_nodes ? t.chunk_nodes : 256;
     c.spin_limit = 1ull << 24;
-    c.donate_min = t.donate_min ? t.donate_min : 64;
+    c.donate_min = t.donate_min;
     c.max_warps = t.max_warps_per_net;
-    c.q_mask = (1ull << qlog2) - 1;
-    c.deadline = ~0ull;  // the boot kernel's deadline; warps of the reducer keep their own
+    dev::queue_begin(c, qlog2, grid * dev::WARPS, queue_runs);
+    c.timeout_ns = timeout_ms * 1000000ull;
     host_ctrl = c;
     CU(cudaMemcpyAsync(ctrl.p, &c, sizeof c, cudaMemcpyHostToDevice, st));
   }
@@ -1227,10 +1264,9 @@ struct Runner {
     heap.alloc(heap_bytes / 8);
     ctrl.alloc(1);
     nets.alloc(progs.size());
-    q.alloc(size_t(1) << qlog2);
+    alloc_queue(size_t(1) << qlog2);
     upload_book();
     prepare_grid(t);
-    size_t qn = size_t(1) << qlog2;
 
     host_nets.assign(progs.size(), dev::NetState{});
     for (size_t i = 0; i < progs.size(); i++) host_nets[i].prog = int(progs[i]);
@@ -1253,12 +1289,7 @@ struct Runner {
     if (mode == HVM64_BATCH_PLAIN && t.chunk_nodes == 0) t.chunk_nodes = 32;
     auto one = [&](unsigned first, unsigned count) {
       // One-net-per-launch runs keep earlier nets' nodes: the bump carries on.
-      reset_ctrl(t, st, qlog2, bump);
-      dev::queue_init_kernel<<<unsigned((qn + 255) / 256), 256, 0, st>>>(q.p, qn);
-      CU(cudaGetLastError());
-      set_deadline(st, timeout_ms);
-      host_ctrl.timeout_ns = timeout_ms * 1000000ull;
-      CU(cudaMemcpyAsync(&ctrl.p->timeout_ns, &host_ctrl.timeout_ns, 8, cudaMemcpyHostToDevice, st));
+      reset_ctrl(t, st, qlog2, bump, timeout_ms);
       CU(cudaEventRecord(e0, st));
       launch(first, count, st);
       CU(cudaEventRecord(e1, st));
@@ -1320,8 +1351,6 @@ struct Runner {
     reduced = true;
   }
 
-  void set_deadline(cudaStream_t st, uint64_t timeout_ms);
-
   // What the device said about its first error (for the error message).
   std::string error_detail;
   void note_error(const dev::Ctrl& h) {
@@ -1366,7 +1395,6 @@ struct Runner {
   }
 
   float run_graph(const hvm64_tuning& t, unsigned qlog2, uint64_t timeout_ms, unsigned first, unsigned count) {
-    size_t qn = size_t(1) << qlog2;
     const unsigned n = unsigned(progs.size());
     std::vector<uint64_t> key = {t.blocks_per_sm, t.chunk_nodes, t.donate_min, qlog2, t.max_warps_per_net, timeout_ms,
                                  first, count, uint64_t(heap.p), uint64_t(q.p), uint64_t(d_defs.p), uint64_t(spill.p),
@@ -1386,10 +1414,8 @@ struct Runner {
       c.heap_bytes = heap_bytes;
       c.chunk_nodes = t.chunk_nodes ? t.chunk_nodes : 256;
       c.spin_limit = 1ull << 24;
-      c.donate_min = t.donate_min ? t.donate_min : 64;
+      c.donate_min = t.donate_min;
       c.max_warps = t.max_warps_per_net;
-      c.q_mask = qn - 1;
-      c.deadline = ~0ull;
       c.timeout_ns = timeout_ms * 1000000ull;
       *pin_ctrl = c;
       CU(cudaHostAlloc(reinterpret_cast<void**>(&pin_params), sizeof(dev::Params), cudaHostAllocDefault));
@@ -1402,10 +1428,6 @@ struct Runner {
       };
       step(cudaMemcpyAsync(nets.p, pin_nets, sizeof(dev::NetState) * n, cudaMemcpyHostToDevice, gs));
       step(cudaMemcpyAsync(ctrl.p, pin_ctrl, sizeof(dev::Ctrl), cudaMemcpyHostToDevice, gs));
-      dev::queue_init_kernel<<<unsigned((qn + 255) / 256), 256, 0, gs>>>(q.p, qn);
-      step(cudaGetLastError());
-      dev::set_deadline_kernel<<<1, 1, 0, gs>>>(ctrl.p, c.timeout_ns);
-      step(cudaGetLastError());
       step(cudaMemcpyToSymbolAsync(dev::g_P, pin_params, sizeof(dev::Params), 0, cudaMemcpyHostToDevice, gs));
       dev::boot_kernel<<<boot_blocks(count, sms), dev::THREADS, dev::SMEM_BYTES, gs>>>(first, count);
       step(cudaGetLastError());
@@ -1424,6 +1446,7 @@ struct Runner {
     cudaEvent_t e0, e1;
     CU(cudaEventCreate(&e0));
     CU(cudaEventCreate(&e1));
+    dev::queue_begin(*pin_ctrl, qlog2, grid * dev::WARPS, queue_runs);  // (the graph copies it to the device)
     CU(cudaEventRecord(e0, gs));
     CU(cudaGraphLaunch(gexec, gs));
     CU(cudaEventRecord(e1, gs));
@@ -1564,10 +1587,6 @@ struct Runner {
   }
 };
 
-namespace dev {
-__global__ void set_deadline_kernel(Ctrl* c, ull timeout_ns) { c->deadline = globaltimer() + timeout_ns; }
-}  // namespace dev
-
 // ===========================================================================
 // Pre-reduce (transform/src/pre_reduce.rs:38-74,136-164) on the device
 // ===========================================================================
@@ -1595,11 +1614,6 @@ PreReduceRun pre_reduce_one(Runner& r, uint32_t id, const hvm64_tuning& tuning, 
   if (ns.status) out.error = r.error_message(ns.status);
   else out.text = r.readback_captured(0);
   return out;
-}
-
-void Runner::set_deadline(cudaStream_t st, uint64_t timeout_ms) {
-  dev::set_deadline_kernel<<<1, 1, 0, st>>>(ctrl.p, uint64_t(timeout_ms) * 1000000ull);
-  CU(cudaGetLastError());
 }
 
 
@@ -1708,14 +1722,15 @@ struct Server {
     c.chunk_nodes = t.chunk_nodes ? t.chunk_nodes : 32;
     c.reuse_mark = c.heap_nodes / 2;
     c.spin_limit = 1ull << 24;
-    c.donate_min = t.donate_min ? t.donate_min : 64;
+    c.donate_min = t.donate_min;
     c.max_warps = t.max_warps_per_net;
-    c.q_mask = qn - 1;
-    c.deadline = ~0ull;
     // a server runs until stopped, or until its lifetime (timeout_ms) ends
     c.timeout_ns = (t.timeout_ms ? t.timeout_ms : 600000ull) * 1000000ull;
+    const unsigned grid = unsigned(sms * reducer_blocks_per_sm(t));
+    uint64_t runs = 0;
+    dev::queue_begin(c, qlog2, grid * dev::WARPS, runs);
     CU(cudaMemcpyAsync(ctrl.p, &c, sizeof c, cudaMemcpyHostToDevice, ks));
-    dev::queue_init_kernel<<<unsigned((qn + 255) / 256), 256, 0, ks>>>(q.p, qn);
+    dev::queue_zero_kernel<<<unsigned((qn + 255) / 256), 256, 0, ks>>>(q.p, qn);
     CU(cudaGetLastError());
     dev::Params p{};
     p.heap = heap.p;
@@ -1734,7 +1749,6 @@ struct Server {
     p.out = d_out;
     p.req_cap = req_cap;
     p.out_cap = out_cap;
-    const unsigned grid = unsigned(sms * reducer_blocks_per_sm(t));
     const uint64_t warps = uint64_t(grid) * dev::WARPS;
     // Node budget for admission: the heap minus what the allocator can hold
     // back while nothing is live (each lane's part-used chunk and unpublished
@@ -2168,6 +2182,7 @@ namespace noalloc {
 constexpr int MAX_DEVICES = 64;
 std::mutex g_setup_mu;
 unsigned char* g_dev_scratch[MAX_DEVICES] = {};
+uint64_t g_queue_runs[MAX_DEVICES] = {};  // runs of the device's scratch queue; held with its DeviceTurn
 
 // The device address of the scratch array on the current device (set-up on
 // the first call per device).
@@ -2218,8 +2233,8 @@ std::string run(const Book& book, const char* name, const hvm64_tuning* tp, hvm6
   cudaStream_t st = 0;
 
   // The array keeps the previous call's contents: everything a run reads
-  // before writing is set here (control block, net record, queue sequence
-  // numbers, Book tables).  Heap nodes are LOCK-filled as they are handed out.
+  // before writing is set here (control block, net record, Book tables), and
+  // the queue's words lie below this run's base.  Heap nodes are LOCK-filled as they are handed out.
   if (defs_b) CU(cudaMemcpyAsync(bk, book.defs.data(), defs_b, cudaMemcpyHostToDevice, st));
   if (ins_b) CU(cudaMemcpyAsync(bk + off_ins, book.instrs.data(), ins_b, cudaMemcpyHostToDevice, st));
   if (lab_b) CU(cudaMemcpyAsync(bk + off_lab, book.labbits.data(), lab_b, cudaMemcpyHostToDevice, st));
@@ -2234,17 +2249,14 @@ std::string run(const Book& book, const char* name, const hvm64_tuning* tp, hvm6
   c.heap_bytes = HEAP_BYTES;
   c.chunk_nodes = t.chunk_nodes ? std::min<uint32_t>(t.chunk_nodes, 64) : CHUNK_NODES;
   c.spin_limit = 1ull << 24;
-  c.donate_min = t.donate_min ? t.donate_min : 64;
+  c.donate_min = t.donate_min;
   c.max_warps = t.max_warps_per_net;
-  c.q_mask = (1ull << QLOG2) - 1;
-  c.deadline = ~0ull;
   c.timeout_ns = timeout_ms * 1000000ull;
+  hvm64_tuning tg = t;
+  if (tg.blocks_per_sm == 0 || tg.blocks_per_sm > 4) tg.blocks_per_sm = 4;
+  unsigned grid = std::min(unsigned(sms * reducer_blocks_per_sm(tg)), MAX_WARPS / unsigned(dev::WARPS));
+  dev::queue_begin(c, QLOG2, grid * dev::WARPS, g_queue_runs[device]);  // (zero when the library is loaded)
   CU(cudaMemcpyAsync(ctrl, &c, sizeof c, cudaMemcpyHostToDevice, st));
-  unsigned qn = 1u << QLOG2;
-  dev::queue_init_kernel<<<(qn + 255) / 256, 256, 0, st>>>(q, qn);
-  CU(cudaGetLastError());
-  dev::set_deadline_kernel<<<1, 1, 0, st>>>(ctrl, c.timeout_ns);
-  CU(cudaGetLastError());
 
   dev::Params p{};
   p.heap = heap;
@@ -2261,9 +2273,6 @@ std::string run(const Book& book, const char* name, const hvm64_tuning* tp, hvm6
   p.spill_cap = SPILL;
   p.gen = gen_matches(book);
   p.ovf_flush = dev::OVF_FLUSH;
-  hvm64_tuning tg = t;
-  if (tg.blocks_per_sm == 0 || tg.blocks_per_sm > 4) tg.blocks_per_sm = 4;
-  unsigned grid = std::min(unsigned(sms * reducer_blocks_per_sm(tg)), MAX_WARPS / unsigned(dev::WARPS));
   upload_params(p, st);
   dev::boot_kernel<<<1, dev::THREADS, dev::SMEM_BYTES, st>>>(0, 1);
   CU(cudaGetLastError());

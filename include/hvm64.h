@@ -55,7 +55,8 @@ typedef struct hvm64_rewrites {
 typedef struct hvm64_tuning {
   uint32_t blocks_per_sm;    /* resident reducer blocks per SM (2 warps each; 0: as many as fit) */
   uint32_t chunk_nodes;      /* nodes a lane takes from the global bump at once */
-  uint32_t donate_min;       /* warp-stack depth above which a warp shares work (the steal threshold) */
+  uint32_t donate_min;       /* waiting redexes from which a warp shares work (the steal threshold; 0: 1 while many
+                              * warps starve, else 64) */
   uint32_t queue_slots_log2; /* global redex-queue capacity, in 32-redex slots (0: 2^20) */
   uint32_t max_warps_per_net; /* warps (plus queued slots) one net's work may spread over (0: no cap) */
   uint32_t flags;            /* HVM64_TUNE_* bits */
@@ -222,7 +223,7 @@ void hvm64_server_free(hvm64_server* server);
  * until the process exits): a 4 MiB region for the Book's device tables, a
  * redex queue of 2^13 slots, overflow stacks for a reducer grid of at most
  * 1184 warps (4 blocks of 2 warps per SM on 148 SMs), and a heap of
- * 3,350,416 nodes.  Lanes take allocator chunks of 8 nodes, so part-used
+ * 3,350,432 nodes.  Lanes take allocator chunks of 8 nodes, so part-used
  * chunks tie up at most 303,104 of them; nodes a warp frees are reused by
  * that warp.  Limits: a Book whose tables exceed 4 MiB is refused with
  * HVM64_ERR_BAD_INPUT; a net that outgrows the heap stops with HVM64_ERR_OOM;
