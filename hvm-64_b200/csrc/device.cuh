@@ -48,7 +48,7 @@ constexpr int HEADROOM = HVM_HEADROOM;  // stack slots kept free for the redexes
 static_assert((SCAP & (SCAP - 1)) == 0 && SCAP >= 64, "SCAP is a power of two, at least 64");
 static_assert(HEADROOM >= 0 && SCAP - HEADROOM >= 32, "a step's window needs SCAP - HEADROOM >= 32");
 constexpr int CHUNK = 32;           // redexes per global-queue slot
-constexpr int POOL = 96;            // per-warp pool of free nodes ready for reuse
+constexpr int POOL = 160;           // per-warp pool of free nodes ready for reuse
 constexpr int FREED_ALONE = 2;      // words an interaction may have freed alone before it looks at their siblings
 constexpr int FAILS = 2;            // wires of an interaction, left as redirects, that it remembers
 constexpr unsigned ICACHE = 32;     // instructions of the step's Def staged in shared memory
@@ -341,7 +341,7 @@ constexpr unsigned RULE_LINK2 = 0, RULE_LINK2_LEN = 2;
 constexpr unsigned RULE_LINK4 = 2, RULE_LINK4_LEN = 4;
 constexpr unsigned RULE_OP = 6, RULE_OP_LEN = 2;
 constexpr unsigned RULE_INS = 8;
-constexpr uint8_t I_OPRED = 9;  // do_op_num on a T_OP node's two wires (device-only instruction)
+// (I_OPRED: do_op_num on a T_OP node's two wires)
 #ifdef __CUDACC__
 __constant__
 #else
@@ -648,10 +648,8 @@ HVM_INL ull alloc(const Ctx c) {
 #ifdef HVM_GEN_INCLUDE
   LS(allocs)++;
 #endif
-  if (c.W->pool_cap) {
-    int k = smem_add_i32(&c.W->pool_n, -1) - 1;
-    if (k >= 0) return c.W->pool[k];
-  }
+  int k = smem_add_i32(&c.W->pool_n, -1) - 1;
+  if (k >= 0) return c.W->pool[k];
   ull b = LS(bnext);
   if (b != LS(bend)) {
     LS(bnext) = b + 1;
@@ -1030,6 +1028,11 @@ HVM_COLD void capture(const Ctx c, ull port, ull trg) {
 //   rule    constructor match, operator, switch: what the operand meets;
 //   link    the operand's target with the other side (linker.rs:25-203).
 //
+// More than half of a Def's instructions build its own nodes, and the encoder
+// knows which (specialise_fresh, host.cpp): those need no take, no match and
+// no general link.  They have kinds of their own (I_CALL to I_FCONST) with a
+// few operations each.
+//
 // Wires an interaction consumes come in pairs, the two words of one consumed
 // node.  The encoder marks the operand that consumes the later one of a pair
 // (INS_A_LAST, INS_B_LAST); the node is reclaimed there, when neither of its
@@ -1087,6 +1090,38 @@ template <unsigned S> HVM_INL void exec_ins(const Ctx c, Exec& x, const DevInstr
     return;
   }
   if (kind == I_CAPTURE) return capture(c, I.port, R[I.a * S]);
+  if (kind >= I_CALL) {  // register b (I_CALL, I_FCTR: none) and, but for I_FLINK, register a hold ports of own nodes
+    if (kind <= I_FCTR) {
+      const ull n = alloc(c);
+      const ull p = mkport(T_CTR, I.lab, n);
+      x.nodes++;
+      if (kind == I_CALL) push(c, I.port, p);
+      else st_gpu(g_P.heap + (paddr(R[I.a * S]) >> 3), p);
+      R[I.b * S] = pvar(n);
+      R[I.c * S] = pvar(n ^ 8);
+      return;
+    }
+    const ull A = R[I.a * S];
+    if (kind == I_FCONST) {
+      st_gpu(g_P.heap + (paddr(A) >> 3), I.port);
+      return;
+    }
+    const ull B = R[I.b * S];
+    ull ap = A;
+    if (ptag(A) == T_RED) {
+      ap = atom_exch(g_P.heap + (A >> 3), P_LOCK);
+      if (ap == P_LOCK) ap = relock(c.net, A);
+      ull ra = pvar(A);
+      if (ptag(ap) == T_VAR) ra = atom_cas(heap_at(c.net, paddr(ap)), pvar(A), B);
+      st_gpu(g_P.heap + (paddr(B) >> 3), ap);
+      if (ra == pvar(A)) wire_done(c, x, A, (I.d & INS_A_LAST) != 0);
+      else wire_failed(c, ap, A, B, x.nf++, (I.d & INS_A_LAST) != 0);
+      return;
+    }
+    if (ptag(A) == T_VAR) st_gpu(g_P.heap + (paddr(A) >> 3), B);
+    st_gpu(g_P.heap + (paddr(B) >> 3), A);
+    return;
+  }
   // take
   const bool isl = kind == I_LINK;
   const ull A = R[I.a * S];

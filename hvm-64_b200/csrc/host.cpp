@@ -609,6 +609,49 @@ struct Encoder {
   }
 };
 
+// Replaces instructions whose operands are known to be fresh (variable ports
+// of nodes the call makes) by their short kinds.  The TrgIds 0 (the argument)
+// and those made from it by a constructor, operator or switch are unknown: at
+// run time they may be wires of consumed nodes.
+static void specialise_fresh(std::vector<RawInstr>& ins, uint32_t ntrgs) {
+  std::vector<uint8_t> fresh(ntrgs, 0);
+  std::vector<int64_t> const_at(ntrgs, -1);  // the I_CONST that makes a TrgId
+  std::vector<uint8_t> drop(ins.size(), 0);
+  for (size_t k = 0; k < ins.size(); k++) {
+    RawInstr& i = ins[k];
+    switch (i.k) {
+      case I_CONST: const_at[i.a] = int64_t(k); break;
+      case I_CTR:
+        if (const_at[i.a] >= 0) {  // no constant is a constructor: never matched
+          i.k = I_CALL;
+          i.port = ins[size_t(const_at[i.a])].port;
+          drop[size_t(const_at[i.a])] = 1;
+        } else if (fresh[i.a]) {
+          i.k = I_FCTR;
+        } else {
+          break;
+        }
+        fresh[i.b] = fresh[i.c] = 1;
+        break;
+      case I_OP: case I_SWITCH: fresh[i.b] = fresh[i.c] = fresh[i.a]; break;
+      case I_OPNUM: fresh[i.c] = fresh[i.a]; break;
+      case I_WIRES: fresh[i.a] = fresh[i.c] = 1; break;
+      case I_LINK:
+        if (fresh[i.a] && !fresh[i.b]) std::swap(i.a, i.b);
+        if (fresh[i.b]) i.k = fresh[i.a] ? I_FFLINK : I_FLINK;
+        break;
+      case I_LINKCONST:
+        if (fresh[i.a]) i.k = I_FCONST;
+        break;
+      default: break;
+    }
+  }
+  size_t n = 0;
+  for (size_t k = 0; k < ins.size(); k++)
+    if (!drop[k]) ins[n++] = ins[k];
+  ins.resize(n);
+}
+
 // Linear-scan renaming: every TrgId is defined once and read once, so a
 // register can be reused right after its single read.
 static uint32_t rename(std::vector<RawInstr>& ins, uint32_t ntrgs) {
@@ -640,12 +683,16 @@ static uint32_t rename(std::vector<RawInstr>& ins, uint32_t ntrgs) {
   for (RawInstr& i : ins) {
     switch (i.k) {
       case I_CONST: def(i.a); break;
-      case I_LINK:
+      case I_LINK: case I_FLINK: case I_FFLINK:
         use(i.a, i.flags, INS_A_LAST);
         use(i.b, i.flags, INS_B_LAST);
         break;
-      case I_LINKCONST: use(i.a, i.flags, INS_A_LAST); break;
-      case I_CTR: case I_OP: case I_SWITCH:
+      case I_LINKCONST: case I_FCONST: use(i.a, i.flags, INS_A_LAST); break;
+      case I_CALL:
+        def(i.b);
+        def(i.c);
+        break;
+      case I_CTR: case I_FCTR: case I_OP: case I_SWITCH:
         use(i.a, i.flags, INS_A_LAST);
         if (i.k == I_CTR) pair(i.b, i.c);
         if (i.k == I_SWITCH) pair(i.c, i.c);  // a wire whose node's other word is free
@@ -682,8 +729,12 @@ static void emit(Book& book, const std::vector<RawInstr>& raw, uint32_t nregs, D
     x.d = r.k == I_WIRES ? uint8_t(r.d) : r.flags;
     x.port = r.port;
     book.instrs.push_back(x);
-    nodes += r.k == I_SWITCH ? 3 : (r.k == I_CTR || r.k == I_OP || r.k == I_OPNUM || r.k == I_WIRES) ? 1 : 0;
-    links += (r.k == I_LINK || r.k == I_LINKCONST) ? 1 : 0;
+    switch (r.k) {
+      case I_SWITCH: nodes += 3; break;
+      case I_CTR: case I_CALL: case I_FCTR: case I_OP: case I_OPNUM: case I_WIRES: nodes++; break;
+      case I_LINK: case I_FLINK: case I_FFLINK: case I_LINKCONST: case I_FCONST: links++; break;
+      default: break;
+    }
   }
   d.nodes = nodes;
   d.redexes = links + nodes;
@@ -702,6 +753,7 @@ static uint32_t encode_net(Book& book, const AstNet& net, DevDef& d) {
     e.small_first = pass == 1;
     e.net(net, 0);
     if (!e.scope.empty()) throw Error(HVM64_ERR_BAD_INPUT, "unbound variables: " + e.scope.begin()->first);
+    specialise_fresh(e.out, e.trgs);
     uint32_t nregs = rename(e.out, e.trgs);
     if (pass == 0 || nregs < best_regs) {
       best = std::move(e.out);
@@ -950,7 +1002,7 @@ std::string compile_defs_cuda(const Book& book) {
     const DevDef& d = book.defs[id];
     for (uint32_t k = 0; k < d.ins_len; k++) {
       const DevInstr& x = book.instrs[d.ins_off + k];
-      if ((x.k == I_CONST || x.k == I_LINKCONST) && (x.port & 7) == T_REF && !(x.port & EXPAND_BIT)) {
+      if ((x.k == I_CONST || x.k == I_LINKCONST || x.k == I_FCONST || x.k == I_CALL) && (x.port & 7) == T_REF && !(x.port & EXPAND_BIT)) {
         uint64_t t = ((x.port & ADDR_MASK) >> 3) - 1;
         if (t < n && t != id) {
           refs[id].push_back(uint32_t(t));
@@ -994,9 +1046,12 @@ std::string compile_defs_cuda(const Book& book) {
       const DevInstr& x = book.instrs[d.ins_off + k];
       switch (x.k) {
         case I_CONST: o += "  " + r(x.a) + " = " + hex(x.port) + ";\n"; break;
-        case I_LINK: o += "  count(c, EX_DLINKS); link_trg(c, " + r(x.a) + ", " + r(x.b) + ");\n"; break;
-        case I_LINKCONST: o += "  count(c, EX_DLINKS); link_trg_port(c, " + r(x.a) + ", " + hex(x.port) + ");\n"; break;
-        case I_CTR:
+        case I_CALL:
+          o += "  do_ctr(c, " + std::to_string(x.lab) + "u, " + hex(x.port) + ", " + r(x.b) + ", " + r(x.c) + ");\n";
+          break;
+        case I_LINK: case I_FLINK: case I_FFLINK: o += "  count(c, EX_DLINKS); link_trg(c, " + r(x.a) + ", " + r(x.b) + ");\n"; break;
+        case I_LINKCONST: case I_FCONST: o += "  count(c, EX_DLINKS); link_trg_port(c, " + r(x.a) + ", " + hex(x.port) + ");\n"; break;
+        case I_CTR: case I_FCTR:
           o += "  do_ctr(c, " + std::to_string(x.lab) + "u, " + r(x.a) + ", " + r(x.b) + ", " + r(x.c) + ");\n";
           break;
         case I_OP:

@@ -41,7 +41,16 @@ inline uint64_t ref_port(uint32_t def_id, uint16_t min_safe) { return port_new(T
 // I_CAPTURE is the whole body of an inert Def (a reference a Book being
 // pre-reduced lacks, transform/src/pre_reduce.rs:89-102): the call's redex
 // (`port`, register a) is recorded for the host instead of expanded.
-enum InstrKind : uint8_t { I_CONST, I_LINK, I_LINKCONST, I_CTR, I_OP, I_OPNUM, I_SWITCH, I_WIRES, I_CAPTURE };
+// I_OPRED is used by the device's rules only.  The kinds from I_CALL on are
+// what other instructions become when the encoder knows that an operand is a
+// port of a node the same call makes (a "fresh" port):
+//   I_CALL    constant + constructor: a new node meets the constant (a redex)
+//   I_FCTR    constructor on a fresh port
+//   I_FLINK   link of anything (a) with a fresh port (b)
+//   I_FFLINK  link of two fresh ports
+//   I_FCONST  constant linked to a fresh port
+enum InstrKind : uint8_t { I_CONST, I_LINK, I_LINKCONST, I_CTR, I_OP, I_OPNUM, I_SWITCH, I_WIRES, I_CAPTURE, I_OPRED,
+                           I_CALL, I_FCTR, I_FLINK, I_FFLINK, I_FCONST };
 
 struct DevInstr {  // 16 bytes
   uint8_t k;

@@ -401,11 +401,16 @@ constexpr unsigned POLL_NS = 1000;  // a waiting warp's pause between two looks 
 #endif
 constexpr int QW = HVM_QW;  // selection window: 32 * QW newest redexes
 
+// Resident blocks per SM.  What bounds a step is its own chain of
+// instructions and round trips, and instruction fetch, not the number of
+// warps that could hide them: 14, 12, 10 and 8 warps an SM measure 360, 361,
+// 362 and 357 ms on a batch of 451 nets and 148, 141, 141 and 140 ms on a sort
+// of 2^15 keys; with 8 to 12 the registers a step needs fit without spills.
 #ifndef HVM_MINB
-#define HVM_MINB 7
+#define HVM_MINB 5
 #endif
 constexpr size_t SMEM_BYTES = sizeof(WarpSmem) * WARPS;
-static_assert(SMEM_BYTES <= 32 * 1024, "seven reducer blocks per SM must fit in shared memory");
+static_assert(HVM_MINB * (SMEM_BYTES + 1024) <= 228 * 1024, "HVM_MINB reducer blocks per SM must fit in shared memory");
 
 __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
   extern __shared__ __align__(16) unsigned char smem_raw[];
