@@ -1484,9 +1484,10 @@ HVM_COLD void interact(const Ctx c, ull a, ull b) {
 // reaches, each redirect chain a Var goes through.  Writes the first `cap`
 // (address, word) pairs to `out` and returns how many there are; `stk` (scap
 // entries) is the depth-first stack.  *deep is set when the stack overflowed
-// (the count is then incomplete).
+// (the count is then incomplete).  A walk of more than `limit` pairs stops soon
+// after them.
 HVM_COLD unsigned gather_walk(unsigned net, ull root, ull* out, unsigned cap, ull* stk,
-                                             unsigned scap, bool* deep) {
+                                             unsigned scap, bool* deep, unsigned limit = ~0u) {
   const ull hb = g_P.heap_bytes;
   unsigned sp = 0, n = 0;
   auto emit = [&](ull w, ull v) {
@@ -1501,7 +1502,7 @@ HVM_COLD unsigned gather_walk(unsigned net, ull root, ull* out, unsigned cap, ul
     return (p >> 48) == 0 && a != 0 && a < hb;
   };
   stk[sp++] = root;
-  while (sp) {
+  while (sp && n <= limit) {
     ull w = stk[--sp];
     ull v = ld_gpu(heap_at(net, w));
     emit(w, v);

@@ -239,53 +239,146 @@ __device__ __noinline__ unsigned serve_gather(WarpSmem& W, unsigned slot, ull ro
 // subtree's count in tcounts (GTASKS per net) for the write pass.  A net
 // whose walk overflows a lane's stack gets count ~0u and is read back from a
 // heap image instead.
-constexpr unsigned GATHER_STACK = 256;
-__global__ void __launch_bounds__(32) gather_kernel(unsigned first, unsigned n, unsigned* counts, const ull* offs,
-                                                    ull* out, unsigned* tcounts) {
-  __shared__ ull tw[GTOP], tv[GTOP], tsz[GTOP];
-  __shared__ unsigned tref[GTOP];
-  __shared__ unsigned char tkind[GTOP];
-  __shared__ unsigned ntop, bad;
+//
+// The count pass gives up a net (GATHER_BIG) with a subtree of more than
+// GATHER_SMALL pairs: its subtrees then get a warp each, which splits them
+// again (big_* kernels).  A walk is a chain of dependent loads, about 0.7 us a
+// word, so the only way to make one large normal form faster is more walks at
+// once: the 459,000 words of a sorted tree of 2^15 keys took one warp 23 ms to
+// count and 17 ms to write (the whole readback 51 ms; 19 ms with this, most of
+// it the text).
+constexpr unsigned GATHER_STACK = 256, GATHER_SMALL = 1024;
+constexpr unsigned GATHER_BIG = ~0u - 1;
+constexpr unsigned GATHER_BIG_NETS = 4096;  // (20 KB each; a run of more nets has a warp for each anyway)
+// The split of one tree, in a block's shared memory.
+struct GatherShared {
+  ull w[GTOP], v[GTOP], sz[GTOP];
+  unsigned ref[GTOP], tc[GTASKS];
+  unsigned char kind[GTOP];
+  unsigned nt, bad, big;
+  __device__ GatherTop top() { return GatherTop{w, v, sz, ref, kind, nt, 0}; }
+};
+// One warp: splits the tree at `root` and counts its subtrees' pairs (tc).
+// Sets G.bad when a walk was too deep, G.big when one passed `limit`.
+__device__ void gather_split(unsigned net, ull root, GatherShared& G, unsigned* tc, ull* stk, unsigned limit) {
   const unsigned lane = threadIdx.x;
-  if (blockIdx.x >= n) return;
-  const unsigned i = first + blockIdx.x;
-  if (out && counts[i] == ~0u) return;
-  unsigned* tc = tcounts + size_t(blockIdx.x) * GTASKS;
-  GatherTop T{tw, tv, tsz, tref, tkind, 0, 0};
   if (lane == 0) {
-    gather_top(i, g_P.nets[i].root, T);
-    ntop = T.nt;
-    bad = 0;
+    GatherTop T = G.top();
+    gather_top(net, root, T);
+    G.nt = T.nt;
+    G.bad = G.big = 0;
   }
   __syncwarp();
-  T.nt = ntop;
-  ull stk[GATHER_STACK];
-  if (!out) {
-    for (unsigned k = lane; k < T.nt; k += 32) {
-      if (tkind[k] != GATHER_SUB) continue;
-      bool deep = false;
-      unsigned c = gather_walk(i, tw[k], nullptr, 0, stk, GATHER_STACK, &deep);
-      tc[tref[k]] = deep ? ~0u : c;
-      if (deep) bad = 1;
-    }
-    __syncwarp();
-    if (lane == 0) {
-      ull total = gather_sizes(T, tc);
-      counts[i] = (bad || total >= 0xFFFFFFFFull) ? ~0u : unsigned(total);
-    }
-    return;
+  for (unsigned k = lane; k < G.nt; k += 32) {
+    if (G.kind[k] != GATHER_SUB) continue;
+    bool deep = false;
+    unsigned c = gather_walk(net, G.w[k], nullptr, 0, stk, GATHER_STACK, &deep, limit);
+    tc[G.ref[k]] = deep ? ~0u : c;
+    if (deep) G.bad = 1;
+    else if (c > limit) G.big = 1;
   }
-  ull* dst = out + 2 * offs[i];
+  __syncwarp();
+}
+// One warp: writes the split tree's pairs at dst.
+__device__ void gather_write(unsigned net, GatherShared& G, const unsigned* tc, ull* dst, ull* stk) {
+  const unsigned lane = threadIdx.x;
   if (lane == 0) {
+    GatherTop T = G.top();
     gather_sizes(T, tc);
     gather_place(T, tc, dst);
   }
   __syncwarp();
-  for (unsigned k = lane; k < T.nt; k += 32) {
-    if (tkind[k] != GATHER_SUB) continue;
+  for (unsigned k = lane; k < G.nt; k += 32) {
+    if (G.kind[k] != GATHER_SUB) continue;
     bool deep = false;
-    gather_walk(i, tw[k], dst + 2 * tsz[k], tc[tref[k]], stk, GATHER_STACK, &deep);
+    gather_walk(net, G.w[k], dst + 2 * G.sz[k], tc[G.ref[k]], stk, GATHER_STACK, &deep);
   }
+}
+__global__ void __launch_bounds__(32) gather_kernel(unsigned first, unsigned n, unsigned* counts, const ull* offs,
+                                                    ull* out, unsigned* tcounts, unsigned limit) {
+  __shared__ GatherShared G;
+  if (blockIdx.x >= n) return;
+  const unsigned i = first + blockIdx.x;
+  unsigned* tc = tcounts + size_t(blockIdx.x) * GTASKS;
+  ull stk[GATHER_STACK];
+  if (!out) {
+    gather_split(i, g_P.nets[i].root, G, tc, stk, limit);
+    if (threadIdx.x == 0) {
+      GatherTop T = G.top();
+      ull total = G.bad || G.big ? 0 : gather_sizes(T, tc);
+      counts[i] = G.bad || total >= GATHER_BIG ? ~0u : G.big ? GATHER_BIG : unsigned(total);
+    }
+    return;
+  }
+  if (counts[i] >= GATHER_BIG || offs[i] == ~0ull) return;
+  if (threadIdx.x == 0) {
+    GatherTop T = G.top();
+    gather_top(i, g_P.nets[i].root, T);
+    G.nt = T.nt;
+  }
+  __syncwarp();
+  gather_write(i, G, tc, out + 2 * offs[i], stk);
+}
+// A big net's split, kept in device memory between the kernels below.
+struct BigNet {
+  ull w[GTOP], v[GTOP], sz[GTOP];
+  unsigned ref[GTOP], tc[GTASKS];
+  unsigned char kind[GTOP];
+  ull task[GTASKS], off[GTASKS];  // each subtree's word and, for the write, its first pair
+  unsigned net, nt, nk, pad;
+  __device__ GatherTop top() { return GatherTop{w, v, sz, ref, kind, nt, nk}; }
+};
+__global__ void __launch_bounds__(32) big_top_kernel(BigNet* big, const unsigned* which) {
+  BigNet& B = big[blockIdx.x];
+  if (threadIdx.x != 0) return;
+  B.net = which[blockIdx.x];
+  GatherTop T = B.top();
+  gather_top(B.net, g_P.nets[B.net].root, T);
+  B.nt = T.nt;
+  B.nk = T.nk;
+  for (unsigned k = 0; k < T.nt; k++)
+    if (T.kind[k] == GATHER_SUB) B.task[T.ref[k]] = T.w[k];
+}
+__global__ void __launch_bounds__(32) big_count_kernel(BigNet* big) {
+  __shared__ GatherShared G;
+  BigNet& B = big[blockIdx.y];
+  if (blockIdx.x >= B.nk) return;
+  ull stk[GATHER_STACK];
+  gather_split(B.net, B.task[blockIdx.x], G, G.tc, stk, ~0u);
+  if (threadIdx.x == 0) {
+    GatherTop T = G.top();
+    ull total = G.bad ? ~0ull : gather_sizes(T, G.tc);
+    B.tc[blockIdx.x] = total >= GATHER_BIG ? ~0u : unsigned(total);
+  }
+}
+__global__ void __launch_bounds__(32) big_sizes_kernel(BigNet* big, unsigned* counts) {
+  BigNet& B = big[blockIdx.x];
+  if (threadIdx.x != 0) return;
+  bool bad = false;
+  for (unsigned k = 0; k < B.nk; k++) bad = bad || B.tc[k] == ~0u;
+  GatherTop T = B.top();
+  ull total = bad ? ~0ull : gather_sizes(T, B.tc);
+  counts[B.net] = total >= GATHER_BIG ? ~0u : unsigned(total);
+}
+__global__ void __launch_bounds__(32) big_place_kernel(BigNet* big, const unsigned* counts, const ull* offs, ull* out) {
+  BigNet& B = big[blockIdx.x];
+  if (threadIdx.x != 0) return;
+  if (counts[B.net] == ~0u) {
+    B.nk = 0;  // read back from a heap image
+    return;
+  }
+  GatherTop T = B.top();
+  gather_place(T, B.tc, out + 2 * offs[B.net]);  // (big_sizes_kernel left the sizes)
+  for (unsigned k = 0; k < T.nt; k++)
+    if (T.kind[k] == GATHER_SUB) B.off[T.ref[k]] = offs[B.net] + T.sz[k];
+}
+__global__ void __launch_bounds__(32) big_write_kernel(BigNet* big, ull* out) {
+  __shared__ GatherShared G;
+  BigNet& B = big[blockIdx.y];
+  if (blockIdx.x >= B.nk) return;
+  ull stk[GATHER_STACK];
+  gather_split(B.net, B.task[blockIdx.x], G, G.tc, stk, ~0u);
+  gather_write(B.net, G, G.tc, out + 2 * B.off[blockIdx.x], stk);
 }
 
 // After a served net's normal form is gathered, nothing refers to its nodes
@@ -1494,6 +1587,8 @@ struct Runner {
   DevBuf<unsigned> d_gcount;
   DevBuf<dev::ull> d_goff, d_gpairs;
   DevBuf<unsigned> d_tcounts;  // gather_kernel's per-subtree counts
+  DevBuf<unsigned> d_which;    // the nets its count pass gave up, and their splits
+  DevBuf<dev::BigNet> d_big;
 
   // Gathers the normal forms of the last run's nets (device-side walk).
   void gather_all() {
@@ -1505,9 +1600,27 @@ struct Runner {
     gcount.assign(n, ~0u);
     d_tcounts.alloc(size_t(std::max(cnt, 1u)) * dev::GTASKS);
     if (cnt) CU(cudaMemcpy(d_gcount.p, gcount.data(), size_t(n) * 4, cudaMemcpyHostToDevice));
-    if (cnt) dev::gather_kernel<<<cnt, 32>>>(first, cnt, d_gcount.p, nullptr, nullptr, d_tcounts.p);
+    const unsigned limit = cnt <= dev::GATHER_BIG_NETS ? dev::GATHER_SMALL : ~0u;
+    if (cnt) dev::gather_kernel<<<cnt, 32>>>(first, cnt, d_gcount.p, nullptr, nullptr, d_tcounts.p, limit);
     CU(cudaGetLastError());
     CU(cudaMemcpy(gcount.data(), d_gcount.p, size_t(n) * 4, cudaMemcpyDeviceToHost));
+    // nets too big for one warp, each of whose subtrees gets one
+    std::vector<unsigned> which;
+    for (unsigned i = first; i < first + cnt; i++)
+      if (gcount[i] == dev::GATHER_BIG) which.push_back(i);
+    const unsigned nbig = unsigned(which.size());
+    if (nbig) {
+      d_which.alloc(nbig);
+      d_big.alloc(nbig);
+      CU(cudaMemcpy(d_which.p, which.data(), size_t(nbig) * 4, cudaMemcpyHostToDevice));
+      h2d += size_t(nbig) * 4;
+      dev::big_top_kernel<<<nbig, 32>>>(d_big.p, d_which.p);
+      dev::big_count_kernel<<<dim3(dev::GTASKS, nbig), 32>>>(d_big.p);
+      dev::big_sizes_kernel<<<nbig, 32>>>(d_big.p, d_gcount.p);
+      CU(cudaGetLastError());
+      CU(cudaMemcpy(gcount.data(), d_gcount.p, size_t(n) * 4, cudaMemcpyDeviceToHost));
+      d2h += size_t(n) * 4;
+    }
     for (unsigned i = 0; i < n; i++)
       if (i < first || i >= first + cnt) gcount[i] = 0;  // not in this run: read back as an error
     goff.resize(n);
@@ -1517,9 +1630,17 @@ struct Runner {
       if (gcount[i] != ~0u) tot += gcount[i];
     }
     d_goff.alloc(n);
-    CU(cudaMemcpy(d_goff.p, goff.data(), size_t(n) * 8, cudaMemcpyHostToDevice));
     d_gpairs.alloc(2 * tot);
-    if (cnt) dev::gather_kernel<<<cnt, 32>>>(first, cnt, d_gcount.p, d_goff.p, d_gpairs.p, d_tcounts.p);
+    // (the one-warp write skips the big nets)
+    std::vector<uint64_t> small_off(goff);
+    for (unsigned i : which) small_off[i] = ~uint64_t(0);
+    CU(cudaMemcpy(d_goff.p, small_off.data(), size_t(n) * 8, cudaMemcpyHostToDevice));
+    if (cnt > nbig) dev::gather_kernel<<<cnt, 32>>>(first, cnt, d_gcount.p, d_goff.p, d_gpairs.p, d_tcounts.p, limit);
+    if (nbig) {
+      CU(cudaMemcpy(d_goff.p, goff.data(), size_t(n) * 8, cudaMemcpyHostToDevice));
+      dev::big_place_kernel<<<nbig, 32>>>(d_big.p, d_gcount.p, d_goff.p, d_gpairs.p);
+      dev::big_write_kernel<<<dim3(dev::GTASKS, nbig), 32>>>(d_big.p, d_gpairs.p);
+    }
     CU(cudaGetLastError());
     std::lock_guard<std::mutex> staged(g_stage.mu);
     uint64_t* pairs = g_stage.reserve(16 * tot);
