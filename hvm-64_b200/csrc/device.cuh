@@ -165,6 +165,11 @@ struct Params {
   unsigned no_expand, capture_cap;
   ull* capture;
   ull rw_limit;
+  // work sharing (see Ctrl, which holds the queue's counters): copies here are
+  // constant-bank operands, where a load would miss L1 after every fence
+  ull q_base, q_mask;
+  unsigned q_warps, donate_min, max_warps;
+  unsigned max_pushes;  // redexes one interaction may push, over all Defs
   unsigned gen;  // 1: the compiled Def functions match the loaded Book (HVM_GEN_INCLUDE builds)
   // serving (all zero for a batch run)
   unsigned serve;

@@ -718,7 +718,7 @@ static void emit(Book& book, const std::vector<RawInstr>& raw, uint32_t nregs, D
                                          std::to_string(MAX_REGS));
   d.ins_off = uint32_t(book.instrs.size());
   d.ins_len = uint32_t(raw.size());
-  d.nregs = nregs;
+  d.nregs = uint16_t(nregs);
   uint32_t nodes = 0, links = 0;
   for (const RawInstr& r : raw) {
     DevInstr x{};
@@ -795,7 +795,7 @@ void Book::load(const AstBook& b, bool inert_missing) {
     d.flags = DEF_INERT;
     d.min_safe = labs[id].min_safe;
     d.lab_off = uint32_t(labbits.size());
-    d.lab_len = uint32_t(labs[id].bits.size());
+    d.lab_len = uint16_t(labs[id].bits.size());
     labbits.insert(labbits.end(), labs[id].bits.begin(), labs[id].bits.end());
     DevInstr x{};
     x.k = I_CAPTURE;
@@ -809,7 +809,7 @@ void Book::load(const AstBook& b, bool inert_missing) {
     encode_net(*this, net, d);
     d.min_safe = labs[id].min_safe;
     d.lab_off = uint32_t(labbits.size());
-    d.lab_len = uint32_t(labs[id].bits.size());
+    d.lab_len = uint16_t(labs[id].bits.size());
     labbits.insert(labbits.end(), labs[id].bits.begin(), labs[id].bits.end());
     defs[id] = d;
   }

@@ -65,10 +65,10 @@ struct DevInstr {  // 16 bytes
 // switch's result is a wire by itself.
 constexpr uint8_t INS_A_LAST = 1, INS_B_LAST = 2;
 
-struct DevDef {  // 36 bytes
+struct DevDef {  // 32 bytes
   uint32_t ins_off, ins_len;
-  uint32_t nregs;
-  uint32_t lab_off, lab_len;  // label bitset words in the shared table
+  uint16_t nregs, lab_len;  // (at most MAX_REGS, and 1024 label bitset words)
+  uint32_t lab_off;         // label bitset words in the shared table
   uint16_t min_safe;
   uint16_t flags;  // DEF_EXPR | DEF_INERT
   uint32_t nodes;  // upper bound on nodes one call allocates
@@ -78,7 +78,7 @@ struct DevDef {  // 36 bytes
 constexpr uint16_t DEF_EXPR = 1;   // an expression program: booting it counts no DREF
 constexpr uint16_t DEF_INERT = 2;  // an inert Def (pre-reduce): its body is one I_CAPTURE
 static_assert(sizeof(DevInstr) == 16, "DevInstr layout");
-static_assert(sizeof(DevDef) == 36, "DevDef layout");
+static_assert(sizeof(DevDef) == 32, "DevDef layout");
 
 // A Def call's registers: up to LOCAL_REGS in the calling thread's local
 // memory; more (up to MAX_REGS, the reach of a DevInstr's one-byte register

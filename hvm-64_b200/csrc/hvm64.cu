@@ -44,13 +44,12 @@ namespace dev {
 // slots, and sharing more work made it slower.)
 //
 // Sequence words: `pos` free for ticket pos, pos + 1 filled, pos + capacity
-// emptied (free for the next lap).  A run's tickets start at Ctrl::q_base, a
+// emptied (free for the next lap).  A run's tickets start at Params::q_base, a
 // multiple of the capacity above every earlier run's, and a word below the
 // base counts as free for its first lap: no run initialises the ring.
 __device__ __forceinline__ ull q_seq(ull pos) {
-  Ctrl* C = g_P.ctrl;
-  ull s = ld_gpu(&g_P.q[pos & C->q_mask].seq);
-  return s < C->q_base ? C->q_base + (pos & C->q_mask) : s;
+  ull s = ld_gpu(&g_P.q[pos & g_P.q_mask].seq);
+  return s < g_P.q_base ? g_P.q_base + (pos & g_P.q_mask) : s;
 }
 // Single-thread reservation by CAS, for a push that must not wait for
 // anything: a full queue returns false at once and the caller keeps the work.
@@ -83,9 +82,9 @@ __device__ bool q_reserve_push(ull& pos) {
 __device__ bool q_ticket_push(unsigned net, ull& pos) {
   Ctrl* C = g_P.ctrl;
   long long used = (long long)(ld_gpu(&C->q_tail) - ld_gpu(&C->q_head));
-  if (used + 40 * (long long)C->q_warps > (long long)C->q_mask) return q_reserve_push(pos);
+  if (used + 40 * (long long)g_P.q_warps > (long long)g_P.q_mask) return q_reserve_push(pos);
   pos = atomicAdd(&C->q_tail, 1ull);
-  if (pos - C->q_base > C->q_mask) {  // past the first lap
+  if (pos - g_P.q_base > g_P.q_mask) {  // past the first lap
     unsigned it = 0;
     while (q_seq(pos) != pos)
       if (!run_spin(net, it)) return false;
@@ -94,11 +93,11 @@ __device__ bool q_ticket_push(unsigned net, ull& pos) {
 }
 __device__ void q_publish(ull pos) {
   __threadfence();
-  st_gpu(&g_P.q[pos & g_P.ctrl->q_mask].seq, pos + 1);
+  st_gpu(&g_P.q[pos & g_P.q_mask].seq, pos + 1);
 }
 __device__ void q_release(ull pos) {
   __threadfence();
-  st_gpu(&g_P.q[pos & g_P.ctrl->q_mask].seq, pos + g_P.ctrl->q_mask + 1);
+  st_gpu(&g_P.q[pos & g_P.q_mask].seq, pos + g_P.q_mask + 1);
 }
 
 // Neither stack of the pushing warp had room (or the pusher has no overflow
@@ -112,7 +111,7 @@ __device__ __noinline__ void push_overflow(unsigned net, ull a, ull b) {
     return;
   }
   atomicAdd(reinterpret_cast<ull*>(&g_P.nets[net].pending), 1ull);
-  Slot* s = &g_P.q[pos & g_P.ctrl->q_mask];
+  Slot* s = &g_P.q[pos & g_P.q_mask];
   st_gpu(reinterpret_cast<ull*>(&s->net), (1ull << 32) | net);
   st_gpu(&s->r[0], a);
   st_gpu(&s->r[1], b);
@@ -136,7 +135,7 @@ __device__ bool donate_vals(ull ra, ull rb, unsigned cnt, int cur) {
   ok = __shfl_sync(0xffffffffu, ok, 0);
   if (!ok) return false;
   pos = shfl(pos, 0);
-  Slot* s = &g_P.q[pos & g_P.ctrl->q_mask];
+  Slot* s = &g_P.q[pos & g_P.q_mask];
   if (lane < cnt) {
     st_gpu(&s->r[2 * lane], ra);
     st_gpu(&s->r[2 * lane + 1], rb);
@@ -642,7 +641,7 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       idle = 0;
       const ull pos = shfl(ticket, 0);
       __threadfence();
-      Slot* s = &g_P.q[pos & C->q_mask];
+      Slot* s = &g_P.q[pos & g_P.q_mask];
       unsigned cnt = 0, net = 0;
       if (lane == 0) {
         ull meta = ld_gpu(reinterpret_cast<const ull*>(&s->net));
@@ -741,11 +740,8 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     // a Def call pushes at most the Def's bound); the rest stay selected-out
     // and go back on the stack below.
     const unsigned nsel32 = n;
-    {
-      unsigned free_slots = unsigned(SCAP) - (top - bot) + n + (W.sp ? W.sp_cap - W.sp_n : 0u);
-      unsigned lim = free_slots / pushes_bound(key);
-      n = max(1u, min(n, lim));
-    }
+    const unsigned free_slots = unsigned(SCAP) - (top - bot) + n + (W.sp ? W.sp_cap - W.sp_n : 0u);
+    if (free_slots / 32u < g_P.max_pushes) n = max(1u, min(n, free_slots / pushes_bound(key)));
     unsigned base = top - w;
     __syncwarp();
     // Entries that stay keep their relative depth (older quarters lower; in a
@@ -787,10 +783,10 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     if (left) {
       int want = 0;
       if (lane == 0) {
-        const unsigned from = C->donate_min ? unsigned(C->donate_min) : starving * 8 >= (long long)C->q_warps ? 1u : 64u;
+        const unsigned from = g_P.donate_min ? g_P.donate_min : starving * 8 >= (long long)g_P.q_warps ? 1u : 64u;
         // a net already spread over max_warps holders (warps and queued
         // slots) gets no more, except to relieve a full overflow stack
-        const ull cap = C->max_warps;
+        const ull cap = g_P.max_warps;
         const bool spread = cap && (ull)ld_gpu64s(&g_P.nets[cur].pending) >= cap;
         want = spread || left < from ? 0 : int(min(max(starving, 0ll), 4ll));
       }
@@ -1015,6 +1011,16 @@ inline void queue_begin(Ctrl& c, unsigned qlog2, unsigned warps, uint64_t& runs)
   c.q_mask = (1ull << qlog2) - 1;
   c.q_warps = warps;
   c.q_base = c.q_head = c.q_tail = ++runs << Q_RUN_BITS;
+}
+// The parameters that repeat a run's control block, and its Book's bound.
+inline void sharing_params(Params& p, const Ctrl& c, const Book& book) {
+  p.q_base = c.q_base;
+  p.q_mask = c.q_mask;
+  p.q_warps = unsigned(c.q_warps);
+  p.donate_min = unsigned(c.donate_min);
+  p.max_warps = unsigned(c.max_warps);
+  p.max_pushes = 4;
+  for (const DevDef& d : book.defs) p.max_pushes = std::max(p.max_pushes, d.redexes);
 }
 
 }  // namespace dev
@@ -1280,6 +1286,7 @@ struct Runner {
     p.rw_limit = rw_limit;
     p.capture = capture.p;
     p.capture_cap = capture.p ? unsigned(capture.n / 2) : 0u;
+    dev::sharing_params(p, host_ctrl, book);
     return p;
   }
 
@@ -1544,7 +1551,8 @@ struct Runner {
     cudaEvent_t e0, e1;
     CU(cudaEventCreate(&e0));
     CU(cudaEventCreate(&e1));
-    dev::queue_begin(*pin_ctrl, qlog2, grid * dev::WARPS, queue_runs);  // (the graph copies it to the device)
+    dev::queue_begin(*pin_ctrl, qlog2, grid * dev::WARPS, queue_runs);  // (the graph copies both to the device)
+    dev::sharing_params(*pin_params, *pin_ctrl, book);
     CU(cudaEventRecord(e0, gs));
     CU(cudaGraphLaunch(gexec, gs));
     CU(cudaEventRecord(e1, gs));
@@ -1880,6 +1888,7 @@ struct Server {
     // back while nothing is live (each lane's part-used chunk and unpublished
     // free list, each warp's reuse pool).
     p.ovf_flush = SERVE_OVF_FLUSH;
+    dev::sharing_params(p, c, book);
     p.gen = gen_matches(book);
     const uint64_t reserve = warps * 32 * (c.chunk_nodes + SERVE_OVF_FLUSH) + warps * dev::POOL;
     if (heap_bytes / 16 <= 2 * reserve)
@@ -2399,6 +2408,7 @@ std::string run(const Book& book, const char* name, const hvm64_tuning* tp, hvm6
   p.spill_cap = SPILL;
   p.gen = gen_matches(book);
   p.ovf_flush = dev::OVF_FLUSH;
+  dev::sharing_params(p, c, book);
   upload_params(p, st);
   dev::boot_kernel<<<1, dev::THREADS, dev::SMEM_BYTES, st>>>(0, 1);
   CU(cudaGetLastError());
