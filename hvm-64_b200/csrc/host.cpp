@@ -838,11 +838,51 @@ uint32_t Book::add_expr(const AstNet& net) {
 // Readback (host/src/readback.rs:23-87)
 // ===========================================================================
 namespace {
+// Variables seen once: the wire's key -> the variable's number.  Open
+// addressing with backward-shift deletion: a normal form inserts and erases
+// every variable once, and a node-based map's allocations were half of the
+// text's time.  Keys are nonzero (word addresses above node 0).
+struct VarMap {
+  std::vector<std::pair<uint64_t, size_t>> slots = std::vector<std::pair<uint64_t, size_t>>(64);
+  size_t used = 0;
+  size_t home(uint64_t key) const { return size_t((key >> 3) * 0x9E3779B97F4A7C15ull >> 20) & (slots.size() - 1); }
+  // The number of `key`, which leaves the map, or -1 after giving it `fresh`.
+  long long take_or_put(uint64_t key, size_t fresh) {
+    const size_t mask = slots.size() - 1;
+    size_t i = home(key);
+    for (; slots[i].first; i = (i + 1) & mask)
+      if (slots[i].first == key) {
+        const long long v = (long long)slots[i].second;
+        for (size_t j = (i + 1) & mask; slots[j].first; j = (j + 1) & mask) {
+          const size_t h = home(slots[j].first);
+          if (((j - h) & mask) >= ((j - i) & mask)) {  // its probe passes the hole
+            slots[i] = slots[j];
+            i = j;
+          }
+        }
+        slots[i].first = 0;
+        used--;
+        return v;
+      }
+    slots[i] = {key, fresh};
+    if (2 * ++used > slots.size()) {
+      std::vector<std::pair<uint64_t, size_t>> old(2 * slots.size());
+      old.swap(slots);
+      for (auto& e : old)
+        if (e.first) {
+          size_t k = home(e.first);
+          while (slots[k].first) k = (k + 1) & (slots.size() - 1);
+          slots[k] = e;
+        }
+    }
+    return -1;
+  }
+};
 struct Reader {
   const Book& book;
   const uint64_t* heap;
   uint64_t words;
-  std::unordered_map<uint64_t, size_t> vars;
+  VarMap vars;
   size_t next_var = 0;
   std::string o;
   // Gathered (address, word) pairs.  The device walk visits words in the
@@ -865,6 +905,15 @@ struct Reader {
     }
     return heap[w];
   }
+  void append_var(size_t id) {  // create_var, in place
+    char buf[16];
+    char* e = buf + sizeof buf;
+    for (id += 1; id > 0; id /= 26) {
+      id -= 1;
+      *--e = char('a' + id % 26);
+    }
+    o.append(e, buf + sizeof buf);
+  }
   bool live_addr(uint64_t p) const { return (p >> 48) == 0 && (p & ADDR_MASK) != 0 && ((p & ADDR_MASK) >> 3) < words; }
   void wire(uint64_t w) { port(load(w), w); }
   void port(uint64_t p, uint64_t from) {
@@ -880,15 +929,8 @@ struct Reader {
             end = t & ADDR_MASK;
           }
         }
-        uint64_t key = std::min(from, end);
-        auto it = vars.find(key);
-        if (it != vars.end()) {
-          o += create_var(it->second);
-          vars.erase(it);
-        } else {
-          vars.emplace(key, next_var);
-          o += create_var(next_var++);
-        }
+        const long long seen = vars.take_or_put(std::min(from, end) | 1, next_var);  // (| 1: never 0)
+        append_var(seen >= 0 ? size_t(seen) : next_var++);
         return;
       }
       case T_REF: {
@@ -900,7 +942,15 @@ struct Reader {
         o += book.names[id];
         return;
       }
-      case T_NUM: o += num_to_string(uint32_t(p)); return;
+      case T_NUM: {
+        if (num_tag(uint32_t(p)) != NT_U24) {
+          o += num_to_string(uint32_t(p));
+          return;
+        }
+        char buf[16];
+        o.append(buf, std::to_chars(buf, buf + sizeof buf, num_payload(uint32_t(p))).ptr);
+        return;
+      }
       case T_OP: {
         uint8_t op = uint8_t(p >> 48);
         uint64_t a = p & ADDR_MASK;
@@ -1171,8 +1221,9 @@ std::string readback_pairs(const Book& book, const uint64_t* pairs, size_t npair
   Reader r{book, nullptr, heap_words, {}, 0, {}};
   r.pairs = pairs;
   r.npairs = npairs;
+  r.o.reserve(6 * npairs);
   r.wire(root);
-  return r.o;
+  return std::move(r.o);
 }
 
 std::vector<ReadbackOut> readback_pairs_many(const Book& book, const uint64_t* pairs, const uint64_t* offsets,
@@ -1208,6 +1259,14 @@ std::vector<ReadbackOut> readback_pairs_many(const Book& book, const uint64_t* p
     return nullptr;
   };
   threads = std::max(1u, std::min<unsigned>(threads, unsigned(std::max<size_t>(n, 1))));
+  // A few short texts: here (a thread with its big stack costs about 80 us;
+  // a walk of a few hundred words nests at most as deep).
+  uint64_t words = 0;
+  for (size_t i = 0; i < n; i++) words += counts[i] == ~0u ? 0 : counts[i];
+  if (words <= SHORT_TEXT_PAIRS) {
+    work(&job);
+    return out;
+  }
   std::vector<pthread_t> ts;
   pthread_attr_t attr;
   pthread_attr_init(&attr);

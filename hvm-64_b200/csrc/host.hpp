@@ -172,6 +172,8 @@ std::string readback(const Book& book, const uint64_t* heap, uint64_t heap_words
 // sharing one variable naming: Host::readback of a net with redexes.
 std::string readback_net(const Book& book, const uint64_t* heap, uint64_t heap_words, uint64_t root,
                          const uint64_t* redexes, size_t nredexes);
+// Normal forms of at most this many pairs are formatted on the calling thread.
+constexpr uint64_t SHORT_TEXT_PAIRS = 1024;
 // Many nets' normal forms from gathered pairs at once, on `threads` host
 // threads: net i's pairs start at pair offsets[i] and number counts[i]
 // (~0u: not gathered, left empty).  A net that fails keeps its message.

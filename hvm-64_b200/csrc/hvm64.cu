@@ -1665,7 +1665,8 @@ struct Runner {
   }
   std::vector<ReadbackOut> gtext;
 
-  std::string readback(unsigned i) {
+  // Net i's text; valid until the next run or readback.
+  const std::string& readback(unsigned i) {
     if (!reduced) throw Error(HVM64_ERR_BAD_INPUT, "net not reduced yet");
     if (i < run_first || i >= run_first + run_count)
       throw Error(HVM64_ERR_BAD_INPUT, "net " + std::to_string(i) + " was not in the last run's range");
@@ -1686,10 +1687,10 @@ struct Runner {
       d2h += used * 16 + 8;
       image_valid = true;
     }
-    std::string out;
-    with_big_stack([&] { out = hvm::readback(book, image.data(), image.size(), host_nets[i].root); });
-    return out;
+    with_big_stack([&] { image_text = hvm::readback(book, image.data(), image.size(), host_nets[i].root); });
+    return image_text;
   }
+  std::string image_text;
 
   // Net i of the last run (a pre-reduce run) with the redexes inert Defs
   // captured: those with an eraser first, each group in capture order.
@@ -1988,7 +1989,9 @@ struct Server {
       std::vector<uint64_t> pairs(2 * size_t(d->pairs));
       memcpy(pairs.data(), out + 2 * size_t(out_cap) * s, pairs.size() * 8);
       uint64_t root = d->root;
-      with_big_stack([&] { text = readback_pairs(book, pairs.data(), d->pairs, heap_bytes / 8, root); });
+      const unsigned n = d->pairs;
+      if (n <= SHORT_TEXT_PAIRS) text = readback_pairs(book, pairs.data(), n, heap_bytes / 8, root);
+      else with_big_stack([&] { text = readback_pairs(book, pairs.data(), n, heap_bytes / 8, root); });
     }
     slot_ticket[s] = 0;
     reserved_nodes -= slot_nodes[s];
@@ -2134,10 +2137,7 @@ int hvm64_net_normal(hvm64_net* net, const hvm64_tuning* t, hvm64_rewrites* out,
 }
 int hvm64_net_readback(hvm64_net* net, char* buf, size_t cap, size_t* len) {
   if (!net) return hvm::set_error(HVM64_ERR_BAD_INPUT, "null argument");
-  std::string s;
-  int rc = guarded([&] { s = net->r.readback(0); });
-  if (rc) return rc;
-  return copy_out(s, buf, cap, len);
+  return guarded([&] { copy_out(net->r.readback(0), buf, cap, len); });
 }
 void hvm64_net_free(hvm64_net* net) { delete net; }
 
@@ -2193,10 +2193,7 @@ int hvm64_batch_normal(hvm64_batch* b, int mode, const hvm64_tuning* t, hvm64_re
 }
 int hvm64_batch_readback(hvm64_batch* b, uint32_t i, char* buf, size_t cap, size_t* len) {
   if (!b || i >= b->r.progs.size()) return hvm::set_error(HVM64_ERR_BAD_INPUT, "bad batch index");
-  std::string s;
-  int rc = guarded([&] { s = b->r.readback(i); });
-  if (rc) return rc;
-  return copy_out(s, buf, cap, len);
+  return guarded([&] { copy_out(b->r.readback(i), buf, cap, len); });
 }
 void hvm64_batch_free(hvm64_batch* b) { delete b; }
 

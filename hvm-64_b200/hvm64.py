@@ -143,9 +143,9 @@ def _check(rc):
 def _read_text(fn, *args):
     n = ctypes.c_size_t()
     _check(fn(*args, None, 0, ctypes.byref(n)))
-    buf = ctypes.create_string_buffer(n.value + 1)
-    _check(fn(*args, buf, n.value + 1, ctypes.byref(n)))
-    return buf.value.decode()
+    buf = bytearray(n.value + 1)
+    _check(fn(*args, (ctypes.c_char * len(buf)).from_buffer(buf), len(buf), ctypes.byref(n)))
+    return str(memoryview(buf)[:n.value], "utf-8")
 
 
 class Book:
