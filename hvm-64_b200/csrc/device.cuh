@@ -1023,7 +1023,9 @@ HVM_COLD void capture(const Ctx c, ull port, ull trg) {
 // usual paths (an out-of-line function per primitive spent most of its
 // instructions saving and restoring registers), and all kinds share one code
 // path for taking a wire, allocating, and linking: the lanes of a step stay
-// together and their memory operations go out together.
+// together and their memory operations go out together.  Against the
+// out-of-line form, on one B200: a sort of 2^15 keys 620 -> 228 ms, a batch of
+// 451 nets 1273 -> 694 ms, 90 -> 63 warp instructions an interaction.
 //
 // Every instruction has the same shape:
 //   take    its operands that are wires, with one exchange each (both in
@@ -1036,7 +1038,8 @@ HVM_COLD void capture(const Ctx c, ull port, ull trg) {
 // More than half of a Def's instructions build its own nodes, and the encoder
 // knows which (specialise_fresh, host.cpp): those need no take, no match and
 // no general link.  They have kinds of their own (I_CALL to I_FCONST) with a
-// few operations each.
+// few operations each (340-690 cycles instead of 1300-2000; a sort of 2^9 keys
+// 20.1 -> 17.9 ms, a batch of 451 nets 369 -> 343 ms).
 //
 // Wires an interaction consumes come in pairs, the two words of one consumed
 // node.  The encoder marks the operand that consumes the later one of a pair
