@@ -837,7 +837,6 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     // Run the redexes: each lane's rule becomes a list of instructions (the
     // Def's, staged, or one of the rules' own) on its shared-memory registers.
     {
-      const unsigned dlen = is_def ? W.idef.ins_len : 0u;
       ull* R = W.regs + lane;
       const DevInstr* ins = W.rules;
       unsigned len = 0, id = 0;
@@ -847,7 +846,7 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
         const unsigned p = classify<32>(c, x, ra, rb, R, id);
         if (p == RUN_DEF) {
           ins = W.icache;
-          len = dlen;
+          len = W.idef.ins_len;
           def = true;
           if (!is_def || W.idef.nregs > SMALL_REGS) {
             run_def(c, id, R[0]);
@@ -870,17 +869,21 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
           len = p >> 8;
         }
       }
-      for (unsigned base = 0;;) {
-        const unsigned end = min(len, base + ICACHE);
-        for (unsigned k = base; k < end; k++) exec_ins<32>(c, x, ins[k - base], R);
-        base += ICACHE;
-        if (base >= dlen) break;
-        // (a Def longer than the staged window: load the next one)
-        __syncwarp();
-        const uint4* src = reinterpret_cast<const uint4*>(g_P.instrs + W.idef.ins_off + base);
-        if (lane < min(dlen - base, ICACHE)) reinterpret_cast<uint4*>(W.icache)[lane] = __ldg(src + lane);
-        if (lane == 0) W.icache_def = ~0u;
-        __syncwarp();
+      // No warp barrier may stand between two instructions of an interaction:
+      // a lane may wait for a word that a later instruction of another lane,
+      // of this warp or of one that waits for this warp, fills (relock,
+      // resolve_redirect_pri), and would wait in vain for a lane held at the
+      // barrier.  So each lane reads what the staged window does not hold.
+      const DevInstr* all = g_P.instrs + (is_def ? W.idef.ins_off : 0u);
+      for (unsigned k = 0; k < len; k++) {
+        DevInstr I;
+        if (k < ICACHE) {
+          I = ins[k];
+        } else {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(all + k));
+          memcpy(&I, &v, sizeof I);
+        }
+        exec_ins<32>(c, x, I, R);
       }
       if (lane < n) {
         exec_counts(c, x, def, W.idef.links);
