@@ -792,6 +792,7 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
         want = spread || left < from ? 0 : int(min(max(starving, 0ll), 4ll));
       }
       want = __shfl_sync(0xffffffffu, want, 0);
+      __syncwarp();  // the selection's writes to the stack, by any lane, before the slots are read from it
       unsigned k = 0;
       for (; k < (sp_high ? 4u : unsigned(want)) && W.sp_n >= 32u; k++) {
         if (!donate_spill(W, cur)) break;
