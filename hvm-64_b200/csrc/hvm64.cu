@@ -625,8 +625,8 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
         // waits; the warp keeps its ticket.
         admitted = __shfl_sync(0xffffffffu, admitted, 0);
         const int net = int(admitted - 1);
+        __syncwarp();  // lane 0's boot pushes are in shared memory before the others read them and their count
         const unsigned total = min(W.ring_cnt, unsigned(SCAP));
-        __syncwarp();
         for (unsigned done = 0; done < total; done += unsigned(CHUNK)) {
           const unsigned k = min(total - done, unsigned(CHUNK));
           ull ra = lane < k ? S[2 * (done + lane)] : 0, rb = lane < k ? S[2 * (done + lane) + 1] : 0;
