@@ -154,16 +154,16 @@ __device__ bool donate(const ull* S, unsigned& bot, unsigned cnt, int cur) {
   bot += cnt;
   return true;
 }
-// The 32 newest redexes of the warp's overflow stack into a slot.
+// The newest redexes of the warp's overflow stack, up to 32, into a slot.
 __device__ bool donate_spill(WarpSmem& W, int cur) {
   const unsigned lane = threadIdx.x & 31;
-  unsigned n = W.sp_n;
-  if (n < 32u) return false;
-  ull i = n - 32u + lane;
-  ull ra = W.sp[2 * i], rb = W.sp[2 * i + 1];
-  if (!donate_vals(ra, rb, 32u, cur)) return false;
+  const unsigned n = W.sp_n, cnt = min(n, 32u);
+  if (!cnt) return false;
+  const ull i = n - cnt + lane;
+  ull ra = lane < cnt ? W.sp[2 * i] : 0, rb = lane < cnt ? W.sp[2 * i + 1] : 0;
+  if (!donate_vals(ra, rb, cnt, cur)) return false;
   __syncwarp();
-  if (lane == 0) W.sp_n = n - 32u;
+  if (lane == 0) W.sp_n = n - cnt;
   __syncwarp();
   return true;
 }
@@ -434,8 +434,8 @@ __device__ __noinline__ void serve_complete(WarpSmem& W, unsigned slot) {
 }
 
 // Take the next request, if the host has written one, and boot it in this
-// warp: its first redexes land in the (empty) ring.  Lane 0 only; returns the
-// slot + 1, or 0.
+// warp: its first redexes land in the (empty) ring and, past its capacity, in
+// the (empty) overflow stack.  Lane 0 only; returns the slot + 1, or 0.
 __device__ __noinline__ unsigned serve_admit(WarpSmem& W, Ctx c) {
   Ctrl* C = g_P.ctrl;
   ull t = ld_gpu(&C->req_tail);
@@ -472,8 +472,6 @@ __device__ __noinline__ unsigned serve_admit(WarpSmem& W, Ctx c) {
   W.ring_base = 0;
   W.ring_cap = SCAP;
   W.ring_cnt = 0;
-  const unsigned sp_cap = W.sp_cap;
-  W.sp_cap = W.sp_n;  // boot redexes past the ring go to the queue
   ull root = alloc(c);
   half_free(c, root ^ 8);  // only the left word is the root wire; the node is reclaimed once it is freed
   if (prog < g_P.ndefs && !(g_P.defs[prog].flags & 1)) W.rw[RW_DREF]++;
@@ -482,7 +480,6 @@ __device__ __noinline__ unsigned serve_admit(WarpSmem& W, Ctx c) {
   root = expand(c, root);
   settle(c);
   st_gpu(&ns.root, root);
-  W.sp_cap = sp_cap;
   return slot + 1;
 }
 
@@ -622,20 +619,22 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       if (got == 2) break;
       if (got == 3) {
         // The booted redexes go to the queue, to this warp or another one that
-        // waits; the warp keeps its ticket.
-        admitted = __shfl_sync(0xffffffffu, admitted, 0);
-        const int net = int(admitted - 1);
-        __syncwarp();  // lane 0's boot pushes are in shared memory before the others read them and their count
-        const unsigned total = min(W.ring_cnt, unsigned(SCAP));
-        for (unsigned done = 0; done < total; done += unsigned(CHUNK)) {
-          const unsigned k = min(total - done, unsigned(CHUNK));
-          ull ra = lane < k ? S[2 * (done + lane)] : 0, rb = lane < k ? S[2 * (done + lane) + 1] : 0;
-          if (!donate_vals(ra, rb, k, net)) {
-            if (lane == 0) run_fail(unsigned(net), HVM64_ERR_QUEUE, 2);
-            break;
-          }
+        // waits; the warp keeps its ticket.  What a full queue does not take
+        // stays this warp's own work, and a slot filled for its ticket
+        // meanwhile waits until that is done.
+        cur = int(__shfl_sync(0xffffffffu, admitted, 0)) - 1;
+        c.net = unsigned(cur);
+        __syncwarp();  // lane 0's boot pushes are visible before the others read them and their count
+        const unsigned booted = W.ring_cnt, spilled = spilled_of(&W, booted);
+        bot = 0;
+        top = min(booted, W.ring_cap);
+        __syncwarp();
+        if (lane == 0) W.sp_n += spilled;
+        __syncwarp();
+        while (donate_spill(W, cur)) {
         }
-        cur = net;  // released above, like a net whose redexes ran out
+        while (top != bot && donate(S, bot, min(top - bot, 32u), cur)) {
+        }
         continue;
       }
       waiting = false;

@@ -38,3 +38,12 @@ def _serve(sizes, tuning, rounds):
 def test_boots_of_many_redexes():
     import hvm64
     _serve(SIZES, hvm64.Tuning(timeout_ms=60000), 20)
+
+
+@pytest.mark.gpu
+def test_boots_that_find_the_queue_full():
+    """A queue of 16 slots and boots of more redexes than it holds slots, or
+    than the warp's stack holds: what the queue does not take is reduced by
+    the warp that booted the request."""
+    import hvm64
+    _serve((1, 33, 513, 600, 1100), hvm64.Tuning(timeout_ms=60000, queue_slots_log2=4), 20)
