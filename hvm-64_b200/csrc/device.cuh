@@ -50,7 +50,6 @@ static_assert(HEADROOM >= 0 && SCAP - HEADROOM >= 32, "a step's window needs SCA
 constexpr int CHUNK = 32;           // redexes per global-queue slot
 constexpr int POOL = 160;           // per-warp pool of free nodes ready for reuse
 constexpr int FREED_ALONE = 2;      // words an interaction may have freed alone before it looks at their siblings
-constexpr int FAILS = 2;            // wires of an interaction, left as redirects, that it remembers
 constexpr unsigned ICACHE = 32;     // instructions of the step's Def staged in shared memory
 constexpr unsigned SMALL_REGS = 10; // Defs with at most this many registers use shared memory
 
@@ -58,6 +57,7 @@ constexpr ull P_ERA = 2;
 constexpr ull P_FREE = 0x8000000000000000ull;
 constexpr ull P_LOCK = 0xFFFFFFFFFFFFFFF0ull;
 constexpr ull P_GONE = 0xFFFFFFFFFFFFFFFFull;
+constexpr ull P_CLAIM = 0xFFFFFFFFFFFFFFF8ull;  // a freed word whose node a lane is about to reclaim (see claim)
 constexpr ull A_MASK = 0x0000FFFFFFFFFFF8ull;
 constexpr ull X_BIT = 1ull << 47;  // expansion-agent Ref ports
 
@@ -388,7 +388,6 @@ struct alignas(16) WarpSmem {
   unsigned cnt[NCOUNT * 32];  // per lane: counts of this step, [counter][lane] (folded into rw)
   ull ovf[32];                // per lane: free list head | pushes since published << 48 (see free_list_push)
   ull fw[FREED_ALONE * 32];   // per lane: words freed alone by the current interaction
-  ull fails[FAILS * 32];      // per lane: consumed wires the current interaction left as redirects
   ull bnext[32], bend[32];    // per lane: pre-LOCKed bump chunk [bnext, bend), node indices
 #ifdef HVM_GEN_INCLUDE
   unsigned allocs[32];        // per lane: nodes allocated (for the DREF statistics)
@@ -667,11 +666,14 @@ HVM_COLD ull alloc_cold(const Ctx c) { return alloc(c); }
 // word, then kept only if its right word is still free -- between the load
 // and the CAS the node may have been reclaimed by the other half's owner,
 // reused, and half-freed again (ABA); then the left word is handed back.
+// (Not LOCK in between: the owner of the other half would take that for a
+// word it linked, see pair_done.)
 HVM_COLD void claim(const Ctx c, ull w, ull other) {
   if (!w || other != P_FREE) return;
   ull l = w & ~8ull;
-  if (hcas(c, l, P_FREE, P_LOCK) != P_FREE) return;
+  if (hcas(c, l, P_FREE, P_CLAIM) != P_FREE) return;
   if (hload(c, l | 8) == P_FREE) {
+    hstore(c, l, P_LOCK);
     hstore(c, l | 8, P_LOCK);
     recycle_stored(c, l);
   } else {
@@ -871,7 +873,7 @@ HVM_COLD void resolve_redirect_pri(const Ctx c, ull ap, ull aw, ull bp) {
       } else {
         half_free(c, xw);
         unsigned it3 = 0;
-        while (hcas(c, yw, P_GONE, P_LOCK) != P_GONE)
+        while (hload(c, yw) != P_GONE)  // (never LOCK meanwhile: see pair_done)
           if (!run_spin(c.net, it3)) return;
         half_free(c, yw);
       }
@@ -1046,40 +1048,33 @@ HVM_COLD void capture(const Ctx c, ull port, ull trg) {
 // (INS_A_LAST, INS_B_LAST); the node is reclaimed there, when neither of its
 // words was left as a redirect (wire_done, wire_failed).
 struct Exec {
-  unsigned nf = 0;  // wires left as redirects so far (the first FAILS of them are in WarpSmem::fails)
+  bool failed = false;  // a wire was left as a redirect
   unsigned anni = 0, oper = 0, eras = 0, nodes = 0;
 };
-#define FAIL(k) (c.W->fails[(k) * 32 + c.lane])
-// Whether this interaction left `w` as a redirect: 1 yes, 0 no, -1 not known
-// (more redirects than are remembered).
-HVM_INL int was_failed(const Ctx c, ull w, unsigned nf) {
-  for (unsigned k = 0; k < unsigned(FAILS) && k < nf; k++)
-    if (FAIL(k) == w) return 1;
-  return nf > unsigned(FAILS) ? -1 : 0;
+// The later wire `w` of a pair was linked, and some wire of this interaction
+// was left as a redirect.  The earlier one's word tells whether it was that
+// one: a linked wire's word still holds the LOCK it was taken with, which
+// nobody else touches any more; a redirect, what it resolves to (P_GONE) and a
+// word freed by whoever followed it are all something else.  (While `w` is
+// not freed nobody reclaims the node, so the word cannot be another's.)
+HVM_COLD void pair_done(const Ctx c, ull w) {
+  if (hload(c, w ^ 8) == P_LOCK) recycle(c, w & ~8ull);
+  else half_free(c, w);  // freed alone; whoever follows the redirect frees the other half
 }
-// The later wire of a pair was linked, and some wire of this interaction was
-// left as a redirect.
-HVM_COLD void pair_done(const Ctx c, ull w, unsigned nf) {
-  int f = was_failed(c, w ^ 8, nf);
-  if (f == 0) recycle(c, w & ~8ull);
-  else if (f == 1) half_free(c, w);  // freed alone; whoever follows the redirect frees the other half
-}  // (not known: the node is given up rather than handed out twice)
-HVM_INL void wire_done(const Ctx c, Exec& x, ull w, bool last) {
+HVM_INL void wire_done(const Ctx c, const Exec& x, ull w, bool last) {
   if (last) {
-    if (x.nf == 0) recycle(c, w & ~8ull);
-    else pair_done(c, w, x.nf);
+    if (!x.failed) recycle(c, w & ~8ull);
+    else pair_done(c, w);
   }
 }
-// The CAS on wire `w`'s other end lost: leave a redirect in `w`.
-HVM_COLD void wire_failed(const Ctx c, ull xp, ull w, ull yp, unsigned nf, bool last) {
+// The CAS on wire `w`'s other end lost: leave a redirect in `w`.  When the
+// earlier wire of its pair was linked, that one's word is freed alone; it is
+// looked at first, while `w` still keeps the node.
+HVM_COLD void wire_failed(const Ctx c, ull xp, ull w, ull yp, bool last) {
+  const bool linked = last && hload(c, w ^ 8) == P_LOCK;
   half_link_failed(c, xp, w, yp);
-  if (!last) {
-    if (nf < unsigned(FAILS)) FAIL(nf) = w;
-  } else if (was_failed(c, w ^ 8, nf) == 0) {
-    half_free(c, w ^ 8);  // the earlier wire was linked: its word is freed alone
-  }
+  if (linked) half_free(c, w ^ 8);
 }
-#undef FAIL
 
 // Instruction `I` on registers R[i * S].
 template <unsigned S> HVM_INL void exec_ins(const Ctx c, Exec& x, const DevInstr I, ull* R) {
@@ -1123,7 +1118,10 @@ template <unsigned S> HVM_INL void exec_ins(const Ctx c, Exec& x, const DevInstr
       if (ptag(ap) == T_VAR) ra = atom_cas(heap_at(c.net, paddr(ap)), pvar(A), B);
       st_gpu(g_P.heap + (paddr(B) >> 3), ap);
       if (ra == pvar(A)) wire_done(c, x, A, (I.d & INS_A_LAST) != 0);
-      else wire_failed(c, ap, A, B, x.nf++, (I.d & INS_A_LAST) != 0);
+      else {
+        x.failed = true;
+        wire_failed(c, ap, A, B, (I.d & INS_A_LAST) != 0);
+      }
       return;
     }
     if (ptag(A) == T_VAR) st_gpu(g_P.heap + (paddr(A) >> 3), B);
@@ -1242,11 +1240,17 @@ template <unsigned S> HVM_INL void exec_ins(const Ctx c, Exec& x, const DevInstr
   }
   if (aw) {
     if (ra == pvar(A)) wire_done(c, x, A, alast);
-    else wire_failed(c, ap, A, bp, x.nf++, alast);
+    else {
+      x.failed = true;
+      wire_failed(c, ap, A, bp, alast);
+    }
   }
   if (bw) {
     if (rb == pvar(B)) wire_done(c, x, B, blast);
-    else wire_failed(c, bp, B, ap, x.nf++, blast);
+    else {
+      x.failed = true;
+      wire_failed(c, bp, B, ap, blast);
+    }
   }
 }
 // The counters of an interaction that ran instructions.

@@ -887,7 +887,7 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       }
       if (lane < n) {
         exec_counts(c, x, def, W.idef.links);
-        if ((other || x.nf) && (W.fw[lane] | W.fw[32 + lane])) settle(c);
+        if ((other || x.failed) && (W.fw[lane] | W.fw[32 + lane])) settle(c);
       }
     }
     __syncwarp();
