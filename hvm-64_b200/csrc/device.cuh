@@ -123,6 +123,27 @@ struct Slot {  // 544 bytes: one chunk of up to 32 redexes of one net
   ull r[2 * CHUNK];
 };
 
+// Host side: the queue's part of a run's control block.  `next` is kept beside
+// the ring: the first ticket of the run to come, above every sequence word that
+// earlier runs left in it (all zero before the first) and a multiple of every
+// capacity.  It moves on by what a run used (queue_end; by more than any run
+// uses until then), so it does not wrap in 2^39 runs.
+constexpr unsigned MAX_QLOG2 = 24;  // the largest capacity
+constexpr unsigned Q_RUN_BITS = 36;
+inline void queue_begin(Ctrl& c, unsigned qlog2, unsigned warps, uint64_t& next) {
+  if (next == 0) next = 1ull << MAX_QLOG2;
+  c.q_mask = (1ull << qlog2) - 1;
+  c.q_warps = warps;
+  c.q_base = c.q_head = c.q_tail = next;
+  next += 1ull << Q_RUN_BITS;
+}
+// `c`: the control block after the run.  Its last words lie at most one lap
+// above its tickets.
+inline void queue_end(const Ctrl& c, uint64_t& next) {
+  const uint64_t used = (c.q_head > c.q_tail ? c.q_head : c.q_tail) + c.q_mask + 1;
+  next = ((used >> MAX_QLOG2) + 1) << MAX_QLOG2;
+}
+
 // Serving: one request (host -> device) and one completion record (device ->
 // host).  Both live in page-locked host memory mapped into the device.
 struct ServeReq {  // 16 bytes

@@ -45,8 +45,9 @@ namespace dev {
 //
 // Sequence words: `pos` free for ticket pos, pos + 1 filled, pos + capacity
 // emptied (free for the next lap).  A run's tickets start at Params::q_base, a
-// multiple of the capacity above every earlier run's, and a word below the
-// base counts as free for its first lap: no run initialises the ring.
+// multiple of the capacity above every word earlier runs left (queue_begin,
+// queue_end), and a word below the base counts as free for its first lap: no
+// run initialises the ring.
 __device__ __forceinline__ ull q_seq(ull pos) {
   ull s = ld_gpu(&g_P.q[pos & g_P.q_mask].seq);
   return s < g_P.q_base ? g_P.q_base + (pos & g_P.q_mask) : s;
@@ -1008,14 +1009,6 @@ __global__ void queue_zero_kernel(Slot* q, ull n) {
   if (i < n) q[i].seq = 0;
 }
 
-// Host side: the queue's part of a run's control block.  `runs` counts the
-// runs that used the queue's buffer (its words were zero before the first).
-constexpr unsigned Q_RUN_BITS = 36;  // tickets one run can hand out: 2^36
-inline void queue_begin(Ctrl& c, unsigned qlog2, unsigned warps, uint64_t& runs) {
-  c.q_mask = (1ull << qlog2) - 1;
-  c.q_warps = warps;
-  c.q_base = c.q_head = c.q_tail = ++runs << Q_RUN_BITS;
-}
 // The parameters that repeat a run's control block, and its Book's bound.
 inline void sharing_params(Params& p, const Ctrl& c, const Book& book) {
   p.q_base = c.q_base;
@@ -1303,7 +1296,7 @@ struct Runner {
 
   // The redex queue: zeroed when it is allocated (its sequence words must lie
   // below every run's q_base), never again.
-  uint64_t queue_runs = 0;
+  uint64_t queue_next = 0;
   void alloc_queue(size_t slots) {
     if (q.p && q.n >= slots) return;
     q.alloc(slots);
@@ -1347,7 +1340,7 @@ struct Runner {
     c.spin_limit = 1ull << 24;
     c.donate_min = t.donate_min;
     c.max_warps = t.max_warps_per_net;
-    dev::queue_begin(c, qlog2, grid * dev::WARPS, queue_runs);
+    dev::queue_begin(c, qlog2, grid * dev::WARPS, queue_next);
     c.timeout_ns = timeout_ms * 1000000ull;
     host_ctrl = c;
     CU(cudaMemcpyAsync(ctrl.p, &c, sizeof c, cudaMemcpyHostToDevice, st));
@@ -1367,7 +1360,7 @@ struct Runner {
     run_count = count;
     DeviceTurn turn(device, t.timeout_ms ? t.timeout_ms : 120000);
     unsigned qlog2 = t.queue_slots_log2 ? t.queue_slots_log2 : DEFAULT_QLOG2;
-    if (qlog2 < 4 || qlog2 > 24) throw Error(HVM64_ERR_BAD_INPUT, "queue_slots_log2 out of range");
+    if (qlog2 < 4 || qlog2 > dev::MAX_QLOG2) throw Error(HVM64_ERR_BAD_INPUT, "queue_slots_log2 out of range");
     h2d = d2h = 0;
     error_detail.clear();
     heap.alloc(heap_bytes / 8);
@@ -1407,6 +1400,7 @@ struct Runner {
       CU(cudaEventElapsedTime(&ms, e0, e1));
       total_ms += ms;
       CU(cudaMemcpy(&host_ctrl, ctrl.p, sizeof host_ctrl, cudaMemcpyDeviceToHost));
+      dev::queue_end(host_ctrl, queue_next);
       h2d += sizeof(dev::Ctrl);
       d2h += sizeof(dev::Ctrl);
       stat_donated += host_ctrl.stat_donated;
@@ -1427,6 +1421,7 @@ struct Runner {
     } else if (t.flags & HVM64_TUNE_GRAPH) {
       total_ms = run_graph(t, qlog2, timeout_ms, first, count);
       CU(cudaMemcpy(&host_ctrl, ctrl.p, sizeof host_ctrl, cudaMemcpyDeviceToHost));
+      dev::queue_end(host_ctrl, queue_next);
       d2h += sizeof(dev::Ctrl);
       stat_donated += host_ctrl.stat_donated;
       stat_spilled += host_ctrl.stat_spilled;
@@ -1555,7 +1550,7 @@ struct Runner {
     cudaEvent_t e0, e1;
     CU(cudaEventCreate(&e0));
     CU(cudaEventCreate(&e1));
-    dev::queue_begin(*pin_ctrl, qlog2, grid * dev::WARPS, queue_runs);  // (the graph copies both to the device)
+    dev::queue_begin(*pin_ctrl, qlog2, grid * dev::WARPS, queue_next);  // (the graph copies both to the device)
     dev::sharing_params(*pin_params, *pin_ctrl, book);
     CU(cudaEventRecord(e0, gs));
     CU(cudaGraphLaunch(gexec, gs));
@@ -1816,7 +1811,7 @@ struct Server {
     out_cap = out_pairs;
     req_cap = 2 * slots + 16;
     unsigned qlog2 = t.queue_slots_log2 ? t.queue_slots_log2 : DEFAULT_QLOG2;
-    if (qlog2 < 4 || qlog2 > 24) throw Error(HVM64_ERR_BAD_INPUT, "queue_slots_log2 out of range");
+    if (qlog2 < 4 || qlog2 > dev::MAX_QLOG2) throw Error(HVM64_ERR_BAD_INPUT, "queue_slots_log2 out of range");
     size_t qn = size_t(1) << qlog2;
     heap.alloc(heap_bytes / 8);
     ctrl.alloc(1);
@@ -1866,8 +1861,8 @@ struct Server {
     // a server runs until stopped, or until its lifetime (timeout_ms) ends
     c.timeout_ns = (t.timeout_ms ? t.timeout_ms : 600000ull) * 1000000ull;
     const unsigned grid = unsigned(sms * reducer_blocks_per_sm(t));
-    uint64_t runs = 0;
-    dev::queue_begin(c, qlog2, grid * dev::WARPS, runs);
+    uint64_t first_run = 0;
+    dev::queue_begin(c, qlog2, grid * dev::WARPS, first_run);
     CU(cudaMemcpyAsync(ctrl.p, &c, sizeof c, cudaMemcpyHostToDevice, ks));
     dev::queue_zero_kernel<<<unsigned((qn + 255) / 256), 256, 0, ks>>>(q.p, qn);
     CU(cudaGetLastError());
@@ -2318,7 +2313,7 @@ namespace noalloc {
 constexpr int MAX_DEVICES = 64;
 std::mutex g_setup_mu;
 unsigned char* g_dev_scratch[MAX_DEVICES] = {};
-uint64_t g_queue_runs[MAX_DEVICES] = {};  // runs of the device's scratch queue; held with its DeviceTurn
+uint64_t g_queue_next[MAX_DEVICES] = {};  // of the device's scratch queue (queue_begin); held with its DeviceTurn
 
 // The device address of the scratch array on the current device (set-up on
 // the first call per device).
@@ -2391,7 +2386,7 @@ std::string run(const Book& book, const char* name, const hvm64_tuning* tp, hvm6
   hvm64_tuning tg = t;
   if (tg.blocks_per_sm == 0 || tg.blocks_per_sm > 4) tg.blocks_per_sm = 4;
   unsigned grid = std::min(unsigned(sms * reducer_blocks_per_sm(tg)), MAX_WARPS / unsigned(dev::WARPS));
-  dev::queue_begin(c, QLOG2, grid * dev::WARPS, g_queue_runs[device]);  // (zero when the library is loaded)
+  dev::queue_begin(c, QLOG2, grid * dev::WARPS, g_queue_next[device]);  // (zero when the library is loaded)
   CU(cudaMemcpyAsync(ctrl, &c, sizeof c, cudaMemcpyHostToDevice, st));
 
   dev::Params p{};
@@ -2419,6 +2414,7 @@ std::string run(const Book& book, const char* name, const hvm64_tuning* tp, hvm6
 
   dev::Ctrl hc{};
   CU(cudaMemcpy(&hc, ctrl, sizeof hc, cudaMemcpyDeviceToHost));
+  dev::queue_end(hc, g_queue_next[device]);
   CU(cudaMemcpy(&hn, ns, sizeof hn, cudaMemcpyDeviceToHost));
   if (hc.error) {
     std::string msg = status_name(hc.error);
