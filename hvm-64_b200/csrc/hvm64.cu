@@ -249,7 +249,10 @@ __device__ __noinline__ unsigned serve_gather(WarpSmem& W, unsigned slot, ull ro
 // it the text).
 constexpr unsigned GATHER_STACK = 256, GATHER_SMALL = 1024;
 constexpr unsigned GATHER_BIG = ~0u - 1;
-constexpr unsigned GATHER_BIG_NETS = 4096;  // (20 KB each; a run of more nets has a warp for each anyway)
+// Big nets of a run that are split (20 KB each).  With more of them the nets'
+// own walks overlap enough: one-warp against split readback of sorts of 2^11
+// keys, 128 nets 11.5 / 9.0 ms, 512 nets 25.3 / 25 ms, 1500 nets 65 / 68 ms.
+constexpr unsigned GATHER_BIG_NETS = 512;
 // The split of one tree, in a block's shared memory.
 struct GatherShared {
   ull w[GTOP], v[GTOP], sz[GTOP];
@@ -1597,8 +1600,22 @@ struct Runner {
   DevBuf<unsigned> d_which;    // the nets its count pass gave up, and their splits
   DevBuf<dev::BigNet> d_big;
 
-  // Gathers the normal forms of the last run's nets (device-side walk).
+  // Gathers the normal forms of the last run's nets (device-side walk).  The
+  // splits of big nets are extra device memory: when something cannot be
+  // allocated beside them, the walk is done again without.
   void gather_all() {
+    unsigned nbig = 0;
+    try {
+      gather_nets(true, nbig);
+    } catch (Error&) {
+      if (!nbig) throw;
+      cudaGetLastError();
+      d_big.release();
+      gather_nets(false, nbig);
+    }
+  }
+  // Sets nbig before it asks for the splits' memory (0 without `split`).
+  void gather_nets(bool split, unsigned& nbig) {
     const unsigned n = unsigned(progs.size()), first = run_first, cnt = run_count;
     DeviceTurn turn(device, 600000);
     upload_params(params(), 0);
@@ -1607,15 +1624,21 @@ struct Runner {
     gcount.assign(n, ~0u);
     d_tcounts.alloc(size_t(std::max(cnt, 1u)) * dev::GTASKS);
     if (cnt) CU(cudaMemcpy(d_gcount.p, gcount.data(), size_t(n) * 4, cudaMemcpyHostToDevice));
-    const unsigned limit = cnt <= dev::GATHER_BIG_NETS ? dev::GATHER_SMALL : ~0u;
-    if (cnt) dev::gather_kernel<<<cnt, 32>>>(first, cnt, d_gcount.p, nullptr, nullptr, d_tcounts.p, limit);
-    CU(cudaGetLastError());
-    CU(cudaMemcpy(gcount.data(), d_gcount.p, size_t(n) * 4, cudaMemcpyDeviceToHost));
+    auto count = [&](unsigned limit) {
+      if (cnt) dev::gather_kernel<<<cnt, 32>>>(first, cnt, d_gcount.p, nullptr, nullptr, d_tcounts.p, limit);
+      CU(cudaGetLastError());
+      CU(cudaMemcpy(gcount.data(), d_gcount.p, size_t(n) * 4, cudaMemcpyDeviceToHost));
+    };
+    count(split ? dev::GATHER_SMALL : ~0u);
     // nets too big for one warp, each of whose subtrees gets one
     std::vector<unsigned> which;
     for (unsigned i = first; i < first + cnt; i++)
       if (gcount[i] == dev::GATHER_BIG) which.push_back(i);
-    const unsigned nbig = unsigned(which.size());
+    if (which.size() > dev::GATHER_BIG_NETS) {
+      which.clear();
+      count(~0u);
+    }
+    nbig = unsigned(which.size());
     if (nbig) {
       d_which.alloc(nbig);
       d_big.alloc(nbig);
@@ -1642,7 +1665,7 @@ struct Runner {
     std::vector<uint64_t> small_off(goff);
     for (unsigned i : which) small_off[i] = ~uint64_t(0);
     CU(cudaMemcpy(d_goff.p, small_off.data(), size_t(n) * 8, cudaMemcpyHostToDevice));
-    if (cnt > nbig) dev::gather_kernel<<<cnt, 32>>>(first, cnt, d_gcount.p, d_goff.p, d_gpairs.p, d_tcounts.p, limit);
+    if (cnt > nbig) dev::gather_kernel<<<cnt, 32>>>(first, cnt, d_gcount.p, d_goff.p, d_gpairs.p, d_tcounts.p, 0);
     if (nbig) {
       CU(cudaMemcpy(d_goff.p, goff.data(), size_t(n) * 8, cudaMemcpyHostToDevice));
       dev::big_place_kernel<<<nbig, 32>>>(d_big.p, d_gcount.p, d_goff.p, d_gpairs.p);
