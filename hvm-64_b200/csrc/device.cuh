@@ -1517,10 +1517,13 @@ HVM_COLD void interact(const Ctx c, ull a, ull b) {
 // reaches, each redirect chain a Var goes through.  Writes the first `cap`
 // (address, word) pairs to `out` and returns how many there are; `stk` (scap
 // entries) is the depth-first stack.  *deep is set when the stack overflowed
-// (the count is then incomplete).  A walk of more than `limit` pairs stops soon
-// after them.
+// (the count is then incomplete).  A walk of more than `limit` pairs stops once
+// it has passed GATHER_SHARE subtrees it still has to come back to, and sets
+// *stopped: a walk with fewer (a list's) has nothing to share.
+constexpr unsigned GATHER_SHARE = 4;
 HVM_COLD unsigned gather_walk(unsigned net, ull root, ull* out, unsigned cap, ull* stk,
-                                             unsigned scap, bool* deep, unsigned limit = ~0u) {
+                                             unsigned scap, bool* deep, unsigned limit = ~0u,
+                                             bool* stopped = nullptr) {
   const ull hb = g_P.heap_bytes;
   unsigned sp = 0, n = 0;
   auto emit = [&](ull w, ull v) {
@@ -1535,7 +1538,11 @@ HVM_COLD unsigned gather_walk(unsigned net, ull root, ull* out, unsigned cap, ul
     return (p >> 48) == 0 && a != 0 && a < hb;
   };
   stk[sp++] = root;
-  while (sp && n <= limit) {
+  while (sp) {
+    if (n > limit && sp >= GATHER_SHARE) {
+      *stopped = true;
+      break;
+    }
     ull w = stk[--sp];
     ull v = ld_gpu(heap_at(net, w));
     emit(w, v);

@@ -241,8 +241,8 @@ __device__ __noinline__ unsigned serve_gather(WarpSmem& W, unsigned slot, ull ro
 // heap image instead.
 //
 // The count pass gives up a net (GATHER_BIG) with a subtree of more than
-// GATHER_SMALL pairs: its subtrees then get a warp each, which splits them
-// again (big_* kernels).  A walk is a chain of dependent loads, about 0.7 us a
+// GATHER_SMALL pairs that splits further (gather_walk): its subtrees then get a
+// warp each, which splits them again (big_* kernels).  A walk is a chain of dependent loads, about 0.7 us a
 // word, so the only way to make one large normal form faster is more walks at
 // once: the 459,000 words of a sorted tree of 2^15 keys took one warp 23 ms to
 // count and 17 ms to write (the whole readback 51 ms; 19 ms with this, most of
@@ -262,7 +262,7 @@ struct GatherShared {
   __device__ GatherTop top() { return GatherTop{w, v, sz, ref, kind, nt, 0}; }
 };
 // One warp: splits the tree at `root` and counts its subtrees' pairs (tc).
-// Sets G.bad when a walk was too deep, G.big when one passed `limit`.
+// Sets G.bad when a walk was too deep, G.big when one stopped past `limit`.
 __device__ void gather_split(unsigned net, ull root, GatherShared& G, unsigned* tc, ull* stk, unsigned limit) {
   const unsigned lane = threadIdx.x;
   if (lane == 0) {
@@ -274,11 +274,11 @@ __device__ void gather_split(unsigned net, ull root, GatherShared& G, unsigned* 
   __syncwarp();
   for (unsigned k = lane; k < G.nt; k += 32) {
     if (G.kind[k] != GATHER_SUB) continue;
-    bool deep = false;
-    unsigned c = gather_walk(net, G.w[k], nullptr, 0, stk, GATHER_STACK, &deep, limit);
+    bool deep = false, stopped = false;
+    unsigned c = gather_walk(net, G.w[k], nullptr, 0, stk, GATHER_STACK, &deep, limit, &stopped);
     tc[G.ref[k]] = deep ? ~0u : c;
     if (deep) G.bad = 1;
-    else if (c > limit) G.big = 1;
+    else if (stopped) G.big = 1;
   }
   __syncwarp();
 }
