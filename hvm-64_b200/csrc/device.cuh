@@ -1291,6 +1291,16 @@ template <unsigned S> HVM_INL void exec_def(const Ctx c, const DevDef& d, ull t0
   for (unsigned k = 0; k < d.ins_len; k++) exec_ins<S>(c, x, ins[k], R);
   exec_counts(c, x, true, d.links);
 }
+// The instructions of Def `id` past those a step stages, for one lane.
+HVM_COLD bool exec_rest(const Ctx c, bool failed, unsigned id, ull* R) {
+  Exec x;
+  x.failed = failed;
+  const DevInstr* ins = g_P.instrs + g_P.defs[id].ins_off;
+  const unsigned len = g_P.defs[id].ins_len;
+  for (unsigned k = ICACHE; k < len; k++) exec_ins<32>(c, x, ins[k], R);
+  exec_counts(c, x, true, 0);
+  return x.failed;
+}
 // A Def call outside a step's shared instruction stream, or one that needs
 // more registers than the warp's shared memory holds for a lane.
 HVM_COLD void exec_large(const Ctx c, const DevDef& d, ull t0) {
