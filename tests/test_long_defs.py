@@ -20,8 +20,8 @@ sys.path.insert(0, HERE)
 CALLS = ("& @f ~ (* z) & @f ~ (z *)", "& @f ~ (z *) & @f ~ (* z)")
 
 
-def _book(fillers, calls, pairs=1):
-    f = "@f = ((u v) (* *))\n" + "& @id ~ (1 *)\n" * fillers + "& @id ~ (u v)\n"
+def _book(fillers, calls, pairs=1, tail="(* *)"):
+    f = f"@f = ((u v) {tail})\n" + "& @id ~ (1 *)\n" * fillers + "& @id ~ (u v)\n"
     main = " ".join(calls.replace("z", f"z{k}") for k in range(pairs))
     return f"@id = (a a)\n{f}@main = * {main}\n"
 
@@ -53,3 +53,22 @@ def test_long_defs_on_the_gpu(fillers, calls, pairs):
     rw = net.normal(hvm64.Tuning(timeout_ms=20000))
     assert net.readback() == want
     assert rw.as_dict() == want_rw
+
+
+# 30, 32, 33 and 35 instructions: both sides of the staged window's end
+EDGE = [(8, "*"), (8, "(* *)"), (9, "*"), (9, "(* *)")]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fillers,tail", EDGE)
+def test_defs_at_the_windows_end(fillers, tail):
+    import hvm64
+    from oracle import oracle
+    for calls in CALLS:
+        src = _book(fillers, calls, 16, tail)
+        want, want_rw, _ = oracle.run_book(src)
+        net = hvm64.Net(hvm64.Book.from_str(src), 256 << 20)
+        net.boot("main")
+        rw = net.normal(hvm64.Tuning(timeout_ms=20000))
+        assert net.readback() == want
+        assert rw.as_dict() == want_rw
