@@ -915,7 +915,13 @@ struct Reader {
     o.append(e, buf + sizeof buf);
   }
   bool live_addr(uint64_t p) const { return (p >> 48) == 0 && (p & ADDR_MASK) != 0 && ((p & ADDR_MASK) >> 3) < words; }
-  void wire(uint64_t w) { port(load(w), w); }
+  unsigned depth = 0, max_depth = ~0u;
+  void wire(uint64_t w) {
+    if (depth == max_depth) throw TextTooDeep{};
+    depth++;
+    port(load(w), w);
+    depth--;
+  }
   void port(uint64_t p, uint64_t from) {
     uint8_t tag = p & 7;
     switch (tag) {
@@ -1217,8 +1223,9 @@ std::string readback_net(const Book& book, const uint64_t* heap, uint64_t heap_w
 }
 
 std::string readback_pairs(const Book& book, const uint64_t* pairs, size_t npairs, uint64_t heap_words,
-                           uint64_t root) {
+                           uint64_t root, unsigned max_depth) {
   Reader r{book, nullptr, heap_words, {}, 0, {}};
+  r.max_depth = max_depth;
   r.pairs = pairs;
   r.npairs = npairs;
   r.o.reserve(6 * npairs);
@@ -1239,6 +1246,8 @@ std::vector<ReadbackOut> readback_pairs_many(const Book& book, const uint64_t* p
     uint64_t heap_words;
     std::vector<ReadbackOut>* out;
     std::atomic<size_t>* next;
+    unsigned max_depth = ~0u;
+    bool too_deep = false;
   } job{&book, pairs, offsets, roots, counts, n, heap_words, &out, &next};
   auto work = [](void* p) -> void* {
     Job* j = static_cast<Job*>(p);
@@ -1248,8 +1257,12 @@ std::vector<ReadbackOut> readback_pairs_many(const Book& book, const uint64_t* p
       ReadbackOut& r = (*j->out)[i];
       if (j->counts[i] == ~0u) continue;  // not gathered: the caller reads it back another way
       try {
-        r.text = readback_pairs(*j->book, j->pairs + 2 * j->offsets[i], j->counts[i], j->heap_words, j->roots[i]);
+        r.text = readback_pairs(*j->book, j->pairs + 2 * j->offsets[i], j->counts[i], j->heap_words, j->roots[i],
+                                j->max_depth);
         r.ok = true;
+      } catch (TextTooDeep&) {
+        j->too_deep = true;
+        break;
       } catch (std::exception& e) {
         r.error = e.what();
       } catch (...) {
@@ -1259,13 +1272,17 @@ std::vector<ReadbackOut> readback_pairs_many(const Book& book, const uint64_t* p
     return nullptr;
   };
   threads = std::max(1u, std::min<unsigned>(threads, unsigned(std::max<size_t>(n, 1))));
-  // A few short texts: here (a thread with its big stack costs about 80 us;
-  // a walk of a few hundred words nests at most as deep).
+  // A few short texts: here (a thread with its big stack costs about 80 us),
+  // unless one nests deeper than the caller's stack may be asked for.
   uint64_t words = 0;
   for (size_t i = 0; i < n; i++) words += counts[i] == ~0u ? 0 : counts[i];
   if (words <= SHORT_TEXT_PAIRS) {
+    job.max_depth = SHORT_TEXT_DEPTH;
     work(&job);
-    return out;
+    if (!job.too_deep) return out;
+    job.max_depth = ~0u;
+    out.assign(n, {});
+    next = 0;
   }
   std::vector<pthread_t> ts;
   pthread_attr_t attr;

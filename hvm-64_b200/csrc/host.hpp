@@ -172,8 +172,11 @@ std::string readback(const Book& book, const uint64_t* heap, uint64_t heap_words
 // sharing one variable naming: Host::readback of a net with redexes.
 std::string readback_net(const Book& book, const uint64_t* heap, uint64_t heap_words, uint64_t root,
                          const uint64_t* redexes, size_t nredexes);
-// Normal forms of at most this many pairs are formatted on the calling thread.
+// Normal forms of at most this many pairs that nest at most this deep are
+// formatted on the calling thread (about 200 bytes of its stack a level).
 constexpr uint64_t SHORT_TEXT_PAIRS = 1024;
+constexpr unsigned SHORT_TEXT_DEPTH = 64;
+struct TextTooDeep {};
 // Many nets' normal forms from gathered pairs at once, on `threads` host
 // threads: net i's pairs start at pair offsets[i] and number counts[i]
 // (~0u: not gathered, left empty).  A net that fails keeps its message.
@@ -184,9 +187,10 @@ struct ReadbackOut {
 std::vector<ReadbackOut> readback_pairs_many(const Book& book, const uint64_t* pairs, const uint64_t* offsets,
                                              const unsigned* counts, const uint64_t* roots, size_t n,
                                              uint64_t heap_words, unsigned threads);
-// The same from the (address, word) pairs a serving reducer gathered.
+// The same from the (address, word) pairs a serving reducer gathered.  Throws
+// TextTooDeep when the text nests deeper than `max_depth`.
 std::string readback_pairs(const Book& book, const uint64_t* pairs, size_t npairs, uint64_t heap_words,
-                           uint64_t root);
+                           uint64_t root, unsigned max_depth = ~0u);
 
 // Book::pre_reduce (transform/src/pre_reduce.rs:38-74,136-164).  Each Def
 // of `ast` not in `skip` is visited in byte order of names and first visits

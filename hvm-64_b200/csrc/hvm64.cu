@@ -2007,8 +2007,15 @@ struct Server {
       memcpy(pairs.data(), out + 2 * size_t(out_cap) * s, pairs.size() * 8);
       uint64_t root = d->root;
       const unsigned n = d->pairs;
-      if (n <= SHORT_TEXT_PAIRS) text = readback_pairs(book, pairs.data(), n, heap_bytes / 8, root);
-      else with_big_stack([&] { text = readback_pairs(book, pairs.data(), n, heap_bytes / 8, root); });
+      bool done = n <= SHORT_TEXT_PAIRS;
+      if (done) {
+        try {
+          text = readback_pairs(book, pairs.data(), n, heap_bytes / 8, root, SHORT_TEXT_DEPTH);
+        } catch (TextTooDeep&) {
+          done = false;
+        }
+      }
+      if (!done) with_big_stack([&] { text = readback_pairs(book, pairs.data(), n, heap_bytes / 8, root); });
     }
     slot_ticket[s] = 0;
     reserved_nodes -= slot_nodes[s];
