@@ -49,6 +49,7 @@ static_assert((SCAP & (SCAP - 1)) == 0 && SCAP >= 64, "SCAP is a power of two, a
 static_assert(HEADROOM >= 0 && SCAP - HEADROOM >= 32, "a step's window needs SCAP - HEADROOM >= 32");
 constexpr int CHUNK = 32;           // redexes per global-queue slot
 constexpr int POOL = 160;           // per-warp pool of free nodes ready for reuse
+constexpr int POOL_BUDGETED = 64;   // and where what a warp holds back comes off a budget or a fixed heap
 constexpr int FREED_ALONE = 2;      // words an interaction may have freed alone before it looks at their siblings
 constexpr unsigned ICACHE = 32;     // instructions of the step's Def staged in shared memory
 constexpr unsigned SMALL_REGS = 10; // Defs with at most this many registers use shared memory
@@ -191,6 +192,7 @@ struct Params {
   ull q_base, q_mask;
   unsigned q_warps, donate_min, max_warps;
   unsigned max_pushes;  // redexes one interaction may push, over all Defs
+  unsigned pool_cap;    // a warp's pool of free nodes: POOL or POOL_BUDGETED
   unsigned gen;  // 1: the compiled Def functions match the loaded Book (HVM_GEN_INCLUDE builds)
   // serving (all zero for a batch run)
   unsigned serve;

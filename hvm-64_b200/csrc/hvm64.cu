@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     W.freed_n = 0;
     W.ring_cnt = 0;
     W.icache_def = ~0u;
-    W.pool_cap = POOL;
+    W.pool_cap = int(g_P.pool_cap);
     W.ring_base = 0;
     W.ring_cap = 0;
     const ull gw = ull(blockIdx.x) * WARPS + (threadIdx.x >> 5);
@@ -911,8 +911,9 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
     // hold LOCK by completed exchanges, or the lane that stored it fenced.)
     {
       int pn = max(W.pool_n, 0);
-      int fn = min(W.freed_n, POOL);
-      int mv = min(fn, POOL - pn);
+      const int cap = W.pool_cap;
+      int fn = min(W.freed_n, cap);
+      int mv = min(fn, cap - pn);
       for (int i = int(lane); i < mv; i += 32) W.pool[pn + i] = W.freed[i];
       for (int i = mv + int(lane); i < fn; i += 32) {
         // pool full: the rest goes to this lane's overflow list
@@ -1014,6 +1015,7 @@ inline void sharing_params(Params& p, const Ctrl& c, const Book& book) {
   p.q_warps = unsigned(c.q_warps);
   p.donate_min = unsigned(c.donate_min);
   p.max_warps = unsigned(c.max_warps);
+  p.pool_cap = POOL;
   p.max_pushes = 4;
   for (const DevDef& d : book.defs) p.max_pushes = std::max(p.max_pushes, d.redexes);
 }
@@ -1907,8 +1909,9 @@ struct Server {
     // free list, each warp's reuse pool).
     p.ovf_flush = SERVE_OVF_FLUSH;
     dev::sharing_params(p, c, book);
+    p.pool_cap = dev::POOL_BUDGETED;
     p.gen = gen_matches(book);
-    const uint64_t reserve = warps * 32 * (c.chunk_nodes + SERVE_OVF_FLUSH) + warps * dev::POOL;
+    const uint64_t reserve = warps * 32 * (c.chunk_nodes + SERVE_OVF_FLUSH) + warps * dev::POOL_BUDGETED;
     if (heap_bytes / 16 <= 2 * reserve)
       throw Error(HVM64_ERR_BAD_INPUT, "heap_bytes too small for a server: its allocator may hold back " +
                                            std::to_string(reserve) + " nodes; give it at least " +
@@ -2430,6 +2433,7 @@ std::string run(const Book& book, const char* name, const hvm64_tuning* tp, hvm6
   p.gen = gen_matches(book);
   p.ovf_flush = dev::OVF_FLUSH;
   dev::sharing_params(p, c, book);
+  p.pool_cap = dev::POOL_BUDGETED;
   upload_params(p, st);
   dev::boot_kernel<<<1, dev::THREADS, dev::SMEM_BYTES, st>>>(0, 1);
   CU(cudaGetLastError());
