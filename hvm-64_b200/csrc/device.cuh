@@ -193,6 +193,7 @@ struct Params {
   unsigned q_warps, donate_min, max_warps;
   unsigned max_pushes;  // redexes one interaction may push, over all Defs
   unsigned pool_cap;    // a warp's pool of free nodes: POOL or POOL_BUDGETED
+  unsigned chunk_shift; // a lane takes at most this fraction (2^-chunk_shift) of the fresh nodes left at once
   unsigned gen;  // 1: the compiled Def functions match the loaded Book (HVM_GEN_INCLUDE builds)
   // serving (all zero for a batch run)
   unsigned serve;
@@ -562,7 +563,9 @@ struct Refill {
   ull node, bnext, bend;
 };
 HVM_COLD Refill alloc_refill(unsigned net, ull* ovf) {
-  if ((*ovf & OVF_ADDR) != 0 || (past_reuse_mark() && free_take(net, ovf))) {
+  const bool own = (*ovf & OVF_ADDR) != 0;
+  const ull used = own ? 0 : ld_gpu(&g_P.ctrl->bump);
+  if (own || (used >= g_P.ctrl->reuse_mark && free_take(net, ovf))) {
     ull a = *ovf & OVF_ADDR, n = *ovf >> 48;
     if (a >= g_P.heap_bytes) {  // links are heap words: checked before the node is handed out
       run_fail(net, HVM64_ERR_BAD_ADDR, a);
@@ -574,7 +577,13 @@ HVM_COLD Refill alloc_refill(unsigned net, ull* ovf) {
     mem_fence();
     return {a, 0, 0};
   }
+  // At most the lane's share of what is left (an eighth of it over all lanes,
+  // see sharing_params): work is shared out to every warp from a few waiting
+  // redexes on, and a full chunk a lane took a tree sum of 2^10 leaves 18 MB of
+  // heap, a sort of 2^9 keys 69 MB.
   ull n = g_P.ctrl->chunk_nodes;
+  const ull share = (g_P.ctrl->heap_nodes - (used < g_P.ctrl->heap_nodes ? used : g_P.ctrl->heap_nodes)) >> g_P.chunk_shift;
+  if (share < n) n = share ? share : 1;
   ull s = atom_add(&g_P.ctrl->bump, n);
   if (s + n > g_P.ctrl->heap_nodes) {
     run_fail(net, HVM64_ERR_OOM, s);

@@ -1016,6 +1016,8 @@ inline void sharing_params(Params& p, const Ctrl& c, const Book& book) {
   p.donate_min = unsigned(c.donate_min);
   p.max_warps = unsigned(c.max_warps);
   p.pool_cap = POOL;
+  p.chunk_shift = 8;  // 8 * lanes, rounded down to a power of two
+  while ((2ull << p.chunk_shift) <= 8ull * 32 * c.q_warps) p.chunk_shift++;
   p.max_pushes = 4;
   for (const DevDef& d : book.defs) p.max_pushes = std::max(p.max_pushes, d.redexes);
 }

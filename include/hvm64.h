@@ -54,7 +54,7 @@ typedef struct hvm64_rewrites {
  * chunk_nodes, donate_min, queue_slots_log2 and max_warps_per_net for a batch. */
 typedef struct hvm64_tuning {
   uint32_t blocks_per_sm;    /* resident reducer blocks per SM (2 warps each; 0: as many as fit) */
-  uint32_t chunk_nodes;      /* nodes a lane takes from the global bump at once */
+  uint32_t chunk_nodes;      /* nodes a lane takes from the global bump at once, at most (fewer as the heap fills) */
   uint32_t donate_min;       /* waiting redexes from which a warp shares work (the steal threshold; 0: 1 while many
                               * warps starve, else 64) */
   uint32_t queue_slots_log2; /* global redex-queue capacity, in 32-redex slots (0: 2^20) */
