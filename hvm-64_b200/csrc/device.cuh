@@ -557,6 +557,7 @@ HVM_COLD bool free_take(unsigned net, ull* ovf) {
   }
   return false;
 }
+constexpr ull CHUNK_LEAST = 8;
 // Pop the lane's free list (or, past the reuse mark, a shared batch) / take
 // a new pre-LOCKed bump chunk.
 struct Refill {
@@ -580,10 +581,12 @@ HVM_COLD Refill alloc_refill(unsigned net, ull* ovf) {
   // At most the lane's share of what is left (an eighth of it over all lanes,
   // see sharing_params): work is shared out to every warp from a few waiting
   // redexes on, and a full chunk a lane took a tree sum of 2^10 leaves 18 MB of
-  // heap, a sort of 2^9 keys 69 MB.
+  // heap, a sort of 2^9 keys 69 MB.  Not below CHUNK_LEAST, where the counter
+  // itself is what a narrow net waits for (a Church tower in 8 MB: 93 ms with
+  // single nodes, 77 ms with full chunks).
   ull n = g_P.ctrl->chunk_nodes;
   const ull share = (g_P.ctrl->heap_nodes - (used < g_P.ctrl->heap_nodes ? used : g_P.ctrl->heap_nodes)) >> g_P.chunk_shift;
-  if (share < n) n = share ? share : 1;
+  if (share < n && n > CHUNK_LEAST) n = share > CHUNK_LEAST ? share : CHUNK_LEAST;
   ull s = atom_add(&g_P.ctrl->bump, n);
   if (s + n > g_P.ctrl->heap_nodes) {
     run_fail(net, HVM64_ERR_OOM, s);
