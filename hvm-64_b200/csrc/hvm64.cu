@@ -1388,9 +1388,14 @@ struct Runner {
     uint64_t timeout_ms = t.timeout_ms ? t.timeout_ms : 120000;
     float total_ms = 0;
     uint64_t bump = 1;
-    // One-net-per-launch runs keep every earlier net's nodes, so they take
-    // small allocator chunks unless told otherwise.
-    if (mode == HVM64_BATCH_PLAIN && t.chunk_nodes == 0) t.chunk_nodes = 32;
+    // One-net-per-launch runs keep every earlier net's nodes and lose what is
+    // left of its lanes' chunks, so they take small chunks unless told
+    // otherwise: at most half of what every lane may lose in every net to come.
+    const bool share_heap = mode == HVM64_BATCH_PLAIN && t.chunk_nodes == 0;
+    auto plain_chunk = [&](uint64_t nets_left) {
+      const uint64_t left = heap_bytes / 16 - std::min(bump, heap_bytes / 16);
+      return uint32_t(std::clamp<uint64_t>(left / (2 * 32 * uint64_t(grid) * dev::WARPS * nets_left), 1, 32));
+    };
     auto one = [&](unsigned first, unsigned count) {
       // One-net-per-launch runs keep earlier nets' nodes: the bump carries on.
       reset_ctrl(t, st, qlog2, bump, timeout_ms);
@@ -1419,7 +1424,10 @@ struct Runner {
       }
     };
     if (mode == HVM64_BATCH_PLAIN) {
-      for (unsigned i = first; i < first + count; i++) one(i, 1);
+      for (unsigned i = first; i < first + count; i++) {
+        if (share_heap) t.chunk_nodes = plain_chunk(first + count - i);
+        one(i, 1);
+      }
     } else if (t.flags & HVM64_TUNE_GRAPH) {
       total_ms = run_graph(t, qlog2, timeout_ms, first, count);
       CU(cudaMemcpy(&host_ctrl, ctrl.p, sizeof host_ctrl, cudaMemcpyDeviceToHost));
