@@ -13,9 +13,11 @@
 //
 // Every wait is bounded: after `spin_limit` polls, or when another lane has
 // already failed, the wait gives up, the run's error word is set and all
-// warps drain and exit.  Every heap address is bounds-checked; an address
-// outside the arena sets HVM64_ERR_BAD_ADDR and is redirected to node 0, so a
-// protocol fault can never become a memory fault.
+// warps drain and exit.  An address is bounds-checked where it is read from the
+// heap to be followed (heap_at, a constructor match, a free list's link); one
+// outside the arena sets HVM64_ERR_BAD_ADDR and is redirected to node 0.  The
+// words of a lane's own nodes and of nodes checked that way are accessed
+// without another check, so a protocol fault cannot become a memory fault.
 #pragma once
 #include <stdint.h>
 #include <stddef.h>
@@ -48,7 +50,9 @@ constexpr int HEADROOM = HVM_HEADROOM;  // stack slots kept free for the redexes
 static_assert((SCAP & (SCAP - 1)) == 0 && SCAP >= 64, "SCAP is a power of two, at least 64");
 static_assert(HEADROOM >= 0 && SCAP - HEADROOM >= 32, "a step's window needs SCAP - HEADROOM >= 32");
 constexpr int CHUNK = 32;           // redexes per global-queue slot
-constexpr int POOL = 160;           // per-warp pool of free nodes ready for reuse
+// Per-warp pool of free nodes ready for reuse.  (With 64 a sort of 2^15 keys takes
+// 92 ms on the device instead of 87, a batch of 451 nets 296 instead of 267.)
+constexpr int POOL = 160;
 constexpr int POOL_BUDGETED = 64;   // and where what a warp holds back comes off a budget or a fixed heap
 constexpr int FREED_ALONE = 2;      // words an interaction may have freed alone before it looks at their siblings
 constexpr unsigned ICACHE = 32;     // instructions of the step's Def staged in shared memory
@@ -71,7 +75,7 @@ struct Ctrl {
   ull heap_bytes;
   ull chunk_nodes;
   ull spin_limit;
-  ull deadline;    // %globaltimer ns
+  ull deadline;    // %globaltimer ns (the host emulation's; reducer warps keep their own, from timeout_ns)
   ull donate_min;
   ull max_warps;   // holders (warps + queued slots) per net beyond which no work is donated; 0: no cap
   ull q_mask;      // queue capacity - 1
@@ -87,7 +91,7 @@ struct Ctrl {
   ull pad3[15];
   ull q_tail;
   ull pad4[15];
-  ull stat_donated, stat_spilled, stat_overflow, stat_taken;
+  ull stat_donated, stat_spilled, stat_overflow, pad10;
   ull stat_steps, stat_lanes, stat_busy_cycles, stat_idle_cycles;
   ull timeout_ns;  // per launch: each warp's deadline is its start + timeout_ns
   ull pad5[7];
@@ -504,12 +508,12 @@ HVM_COLD void push_overflow(unsigned net, ull a, ull b);
 // published in bits 48-63.
 //
 // Free nodes move between warps through one shared stack of batches, once
-// the heap is past its reuse mark (Ctrl::reuse_mark; a batch run sets it at
-// half the heap, a server at 0): a lane's list is published whole once it
-// holds Params::ovf_flush nodes (OVF_FLUSH for a batch, 32 for a server, which
-// keeps fewer nodes stranded per lane), the batch's head node linking the next batch through
-// its right word, and a lane whose list is empty takes a batch before it
-// takes fresh nodes from the bump pointer.  Below the mark, allocation stays
+// the heap is past its reuse mark (Ctrl::reuse_mark: half the heap): a lane's
+// list is published whole once it holds Params::ovf_flush nodes (OVF_FLUSH for
+// a batch, 32 for a server, which keeps fewer nodes stranded per lane), the
+// batch's head node linking the next batch through its right word, and a lane
+// whose list is empty takes a batch before it takes fresh nodes from the bump
+// pointer.  Below the mark, allocation stays
 // on the bump pointer and the lanes' own lists (no shared traffic).  The top
 // word carries a push/pop count above the address bits, so a pop whose
 // batch was taken and republished meanwhile fails its CAS (ABA).
@@ -605,11 +609,10 @@ HVM_INL void free_list_push(unsigned net, ull* ovf, ull node) {
 }
 
 // ---- the runtime proper ------------------------------------------------------
-// Every rule, link operation and VM instruction is one out-of-line function
-// over a three-word context (warp state, lane, net).  A lane's mutable state
-// (freed-word slots, bump chunk) lives in its warp's shared memory, so these
-// functions keep nothing in local memory and each exists once in the binary:
-// the hot code fits the instruction cache.
+// Everything works on a three-word context (warp state, lane, net).  A lane's
+// mutable state (freed-word slots, bump chunk) lives in its warp's shared
+// memory.  The usual paths are inlined once into the reducer's step (exec_ins);
+// the others are out-of-line functions.
 struct Ctx {
   WarpSmem* W;
   unsigned lane;
@@ -833,24 +836,6 @@ HVM_COLD void half_link_wire_port(const Ctx c, ull ap, ull aw, ull bp) {
     half_free(c, aw);
   }
 }
-HVM_COLD void link_wire_wire(const Ctx c, ull aw, ull bw) {
-  // Both words belong to nodes this interaction consumes, so no other lane
-  // takes them: the two exchanges go out together (one round trip instead of
-  // two) and give the values the reference's take-one-then-the-other does; a
-  // word its creator has not written yet (LOCK) is waited for after both.
-  ull ap = hswap(c, aw, P_LOCK);
-  ull bp = hswap(c, bw, P_LOCK);
-  if (ap == P_LOCK) ap = relock(c.net, aw);
-  if (bp == P_LOCK) bp = relock(c.net, bw);
-  if (principal(ap) && principal(bp)) {
-    half_free(c, aw);
-    half_free(c, bw);
-    redux(c, ap, bp);
-  } else {
-    half_link_wire_port(c, ap, aw, bp);
-    half_link_wire_port(c, bp, bw, ap);
-  }
-}
 // link_wire_port for a wire whose target `ap` was already taken (locked).
 HVM_COLD void link_locked_wire_port(const Ctx c, ull aw, ull ap, ull bp) {
   if (principal(ap) && principal(bp)) {
@@ -925,6 +910,24 @@ HVM_COLD void resolve_redirect_pri(const Ctx c, ull ap, ull aw, ull bp) {
 HVM_INL void link_trg_port(const Ctx c, ull a, ull b) {
   if (trg_is_wire(a)) link_wire_port(c, a, b);
   else link_port_port(c, a, b);
+}
+HVM_COLD void link_wire_wire(const Ctx c, ull aw, ull bw) {
+  // Both words belong to nodes this interaction consumes, so no other lane
+  // takes them: the two exchanges go out together (one round trip instead of
+  // two) and give the values the reference's take-one-then-the-other does; a
+  // word its creator has not written yet (LOCK) is waited for after both.
+  ull ap = hswap(c, aw, P_LOCK);
+  ull bp = hswap(c, bw, P_LOCK);
+  if (ap == P_LOCK) ap = relock(c.net, aw);
+  if (bp == P_LOCK) bp = relock(c.net, bw);
+  if (principal(ap) && principal(bp)) {
+    half_free(c, aw);
+    half_free(c, bw);
+    redux(c, ap, bp);
+  } else {
+    half_link_wire_port(c, ap, aw, bp);
+    half_link_wire_port(c, bp, bw, ap);
+  }
 }
 HVM_COLD void link_trg(const Ctx c, ull a, ull b) {
   bool aw = trg_is_wire(a), bw = trg_is_wire(b);

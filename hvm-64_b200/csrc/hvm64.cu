@@ -970,7 +970,6 @@ __global__ void __launch_bounds__(THREADS) boot_kernel(unsigned first, unsigned 
       ull root = alloc(c);
       unsigned prog = unsigned(ns.prog);
       if (prog < g_P.ndefs && !(g_P.defs[prog].flags & 1)) W.rw[RW_DREF]++;
-      // Small Defs use register slots 0, 32, 64, ... of W.regs (lane 0's column).
       run_def(c, prog, pvar(root));
       settle(c);
       if (!g_P.no_expand) {
@@ -1176,11 +1175,10 @@ void upload_params(const dev::Params& p, cudaStream_t st) {
 
 }  // namespace
 
-// Default redex-queue capacity: 2^20 slots (570 MB).  A warp whose stack is
-// full ships redexes to the queue one per slot in the middle of a step, and a
-// warp that finds the queue full waits for consumers; when every warp waits
-// like that at once the run stops with TIMEOUT, so the queue is sized for
-// bursts from Defs that create many redexes at once.
+// Default redex-queue capacity: 2^20 slots (570 MB).  A warp whose stacks are
+// both full ships redexes to the queue one per slot in the middle of a step,
+// and a run whose queue has no room for one stops with QUEUE, so the queue is
+// sized for bursts from Defs that create many redexes at once.
 constexpr unsigned DEFAULT_QLOG2 = 20;
 
 // Host staging for gathered normal forms, shared by the process's runs (one
@@ -1482,10 +1480,10 @@ struct Runner {
   }
   std::string error_message(int code) const { return std::string(status_name(code)) + error_detail; }
 
-  // A persistent run as one CUDA graph: net records, control block, queue
-  // init, deadline, launch parameters, boot and reduce, captured once per
-  // configuration and replayed by later runs.  Its host sources are
-  // page-locked copies that stay valid while the graph does.
+  // A persistent run as one CUDA graph: net records, control block, launch
+  // parameters, boot and reduce, captured once per configuration and replayed
+  // by later runs.  Its host sources are page-locked copies that stay valid
+  // while the graph does.
   cudaStream_t gs = nullptr;
   cudaGraphExec_t gexec = nullptr;
   std::vector<uint64_t> gkey;
