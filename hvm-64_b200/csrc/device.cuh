@@ -55,6 +55,7 @@ constexpr int CHUNK = 32;           // redexes per global-queue slot
 constexpr int POOL = 160;
 constexpr int POOL_BUDGETED = 64;   // and where what a warp holds back comes off a budget or a fixed heap
 constexpr int FREED_ALONE = 2;      // words an interaction may have freed alone before it looks at their siblings
+constexpr int FAILS = 2;            // wires of an interaction, left as redirects, that it remembers
 constexpr unsigned ICACHE = 32;     // instructions of the step's Def staged in shared memory
 constexpr unsigned SMALL_REGS = 10; // Defs with at most this many registers use shared memory
 
@@ -416,6 +417,7 @@ struct alignas(16) WarpSmem {
   unsigned cnt[NCOUNT * 32];  // per lane: counts of this step, [counter][lane] (folded into rw)
   ull ovf[32];                // per lane: free list head | pushes since published << 48 (see free_list_push)
   ull fw[FREED_ALONE * 32];   // per lane: words freed alone by the current interaction
+  ull fails[FAILS * 32];      // per lane: the first consumed wires the current interaction left as redirects
   ull bnext[32], bend[32];    // per lane: pre-LOCKed bump chunk [bnext, bend), node indices
 #ifdef HVM_GEN_INCLUDE
   unsigned allocs[32];        // per lane: nodes allocated (for the DREF statistics)
@@ -705,7 +707,7 @@ HVM_COLD ull alloc_cold(const Ctx c) { return alloc(c); }
 // and the CAS the node may have been reclaimed by the other half's owner,
 // reused, and half-freed again (ABA); then the left word is handed back.
 // (Not LOCK in between: the owner of the other half would take that for a
-// word it linked, see pair_done.)
+// word it linked, see was_linked.)
 HVM_COLD void claim(const Ctx c, ull w, ull other) {
   if (!w || other != P_FREE) return;
   ull l = w & ~8ull;
@@ -893,7 +895,7 @@ HVM_COLD void resolve_redirect_pri(const Ctx c, ull ap, ull aw, ull bp) {
       } else {
         half_free(c, xw);
         unsigned it3 = 0;
-        while (hload(c, yw) != P_GONE)  // (never LOCK meanwhile: see pair_done)
+        while (hload(c, yw) != P_GONE)  // (never LOCK meanwhile: see was_linked)
           if (!run_spin(c.net, it3)) return;
         half_free(c, yw);
       }
@@ -1086,33 +1088,44 @@ HVM_COLD void capture(const Ctx c, ull port, ull trg) {
 // (INS_A_LAST, INS_B_LAST); the node is reclaimed there, when neither of its
 // words was left as a redirect (wire_done, wire_failed).
 struct Exec {
-  bool failed = false;  // a wire was left as a redirect
+  unsigned nf = 0;  // wires left as redirects so far (the first FAILS of them are in WarpSmem::fails)
   unsigned anni = 0, oper = 0, eras = 0, nodes = 0;
 };
+#define FAIL(k) (c.W->fails[(k) * 32 + c.lane])
+// Whether this interaction, which has left `nf` wires as redirects, linked the
+// wire `w`.  Past the wires it remembers the word tells: a linked wire's still
+// holds the LOCK it was taken with, which nobody else touches any more; a
+// redirect, what it resolves to (P_GONE) and a word freed by whoever followed
+// it are all something else.  Asked while the node's other word is this
+// lane's: nobody reclaims the node, so the word cannot be another's.  (Always
+// reading the word: a tree sum of 2^18 leaves 3.39 -> 3.47 ms.)
+HVM_INL bool was_linked(const Ctx c, ull w, unsigned nf) {
+  for (unsigned k = 0; k < unsigned(FAILS) && k < nf; k++)
+    if (FAIL(k) == w) return false;
+  return nf <= unsigned(FAILS) || hload(c, w) == P_LOCK;
+}
 // The later wire `w` of a pair was linked, and some wire of this interaction
-// was left as a redirect.  The earlier one's word tells whether it was that
-// one: a linked wire's word still holds the LOCK it was taken with, which
-// nobody else touches any more; a redirect, what it resolves to (P_GONE) and a
-// word freed by whoever followed it are all something else.  (While `w` is
-// not freed nobody reclaims the node, so the word cannot be another's.)
-HVM_COLD void pair_done(const Ctx c, ull w) {
-  if (hload(c, w ^ 8) == P_LOCK) recycle(c, w & ~8ull);
+// was left as a redirect.
+HVM_COLD void pair_done(const Ctx c, ull w, unsigned nf) {
+  if (was_linked(c, w ^ 8, nf)) recycle(c, w & ~8ull);
   else half_free(c, w);  // freed alone; whoever follows the redirect frees the other half
 }
 HVM_INL void wire_done(const Ctx c, const Exec& x, ull w, bool last) {
   if (last) {
-    if (!x.failed) recycle(c, w & ~8ull);
-    else pair_done(c, w);
+    if (x.nf == 0) recycle(c, w & ~8ull);
+    else pair_done(c, w, x.nf);
   }
 }
-// The CAS on wire `w`'s other end lost: leave a redirect in `w`.  When the
-// earlier wire of its pair was linked, that one's word is freed alone; it is
-// looked at first, while `w` still keeps the node.
-HVM_COLD void wire_failed(const Ctx c, ull xp, ull w, ull yp, bool last) {
-  const bool linked = last && hload(c, w ^ 8) == P_LOCK;
+// The CAS on wire `w`'s other end lost: leave a redirect in `w`, the
+// interaction's `nf`-th.  When the earlier wire of its pair was linked, that
+// one's word is freed alone.
+HVM_COLD void wire_failed(const Ctx c, ull xp, ull w, ull yp, unsigned nf, bool last) {
+  const bool linked = last && was_linked(c, w ^ 8, nf);
+  if (nf < unsigned(FAILS)) FAIL(nf) = w;
   half_link_failed(c, xp, w, yp);
   if (linked) half_free(c, w ^ 8);
 }
+#undef FAIL
 
 // Instruction `I` on registers R[i * S].
 template <unsigned S> HVM_INL void exec_ins(const Ctx c, Exec& x, const DevInstr I, ull* R) {
@@ -1156,10 +1169,7 @@ template <unsigned S> HVM_INL void exec_ins(const Ctx c, Exec& x, const DevInstr
       if (ptag(ap) == T_VAR) ra = atom_cas(heap_at(c.net, paddr(ap)), pvar(A), B);
       st_gpu(g_P.heap + (paddr(B) >> 3), ap);
       if (ra == pvar(A)) wire_done(c, x, A, (I.d & INS_A_LAST) != 0);
-      else {
-        x.failed = true;
-        wire_failed(c, ap, A, B, (I.d & INS_A_LAST) != 0);
-      }
+      else wire_failed(c, ap, A, B, x.nf++, (I.d & INS_A_LAST) != 0);
       return;
     }
     if (ptag(A) == T_VAR) st_gpu(g_P.heap + (paddr(A) >> 3), B);
@@ -1278,17 +1288,11 @@ template <unsigned S> HVM_INL void exec_ins(const Ctx c, Exec& x, const DevInstr
   }
   if (aw) {
     if (ra == pvar(A)) wire_done(c, x, A, alast);
-    else {
-      x.failed = true;
-      wire_failed(c, ap, A, bp, alast);
-    }
+    else wire_failed(c, ap, A, bp, x.nf++, alast);
   }
   if (bw) {
     if (rb == pvar(B)) wire_done(c, x, B, blast);
-    else {
-      x.failed = true;
-      wire_failed(c, bp, B, ap, blast);
-    }
+    else wire_failed(c, bp, B, ap, x.nf++, blast);
   }
 }
 // The counters of an interaction that ran instructions.
@@ -1309,14 +1313,14 @@ template <unsigned S> HVM_INL void exec_def(const Ctx c, const DevDef& d, ull t0
   exec_counts(c, x, true, d.links);
 }
 // The instructions of Def `id` past those a step stages, for one lane.
-HVM_COLD bool exec_rest(const Ctx c, bool failed, unsigned id, ull* R) {
+HVM_COLD unsigned exec_rest(const Ctx c, unsigned nf, unsigned id, ull* R) {
   Exec x;
-  x.failed = failed;
+  x.nf = nf;
   const DevInstr* ins = g_P.instrs + g_P.defs[id].ins_off;
   const unsigned len = g_P.defs[id].ins_len;
   for (unsigned k = ICACHE; k < len; k++) exec_ins<32>(c, x, ins[k], R);
   exec_counts(c, x, true, 0);
-  return x.failed;
+  return x.nf;
 }
 // A Def call outside a step's shared instruction stream, or one that needs
 // more registers than the warp's shared memory holds for a lane.

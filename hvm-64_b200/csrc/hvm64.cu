@@ -883,10 +883,10 @@ __global__ void __launch_bounds__(THREADS, HVM_MINB) reduce_kernel() {
       // 98.9 -> 104.4 ms).
       const unsigned window = min(len, ICACHE);
       for (unsigned k = 0; k < window; k++) exec_ins<32>(c, x, ins[k], R);
-      if (len > ICACHE) x.failed = exec_rest(c, x.failed, id, R);
+      if (len > ICACHE) x.nf = exec_rest(c, x.nf, id, R);
       if (lane < n) {
         exec_counts(c, x, def, W.idef.links);
-        if ((other || x.failed) && (W.fw[lane] | W.fw[32 + lane])) settle(c);
+        if ((other || x.nf) && (W.fw[lane] | W.fw[32 + lane])) settle(c);
       }
     }
     __syncwarp();
